@@ -1,12 +1,10 @@
 """Scheduling autotuner for the batched grid / degrid calls.
 
 The batched calls (``device.grid`` / ``device.degrid`` with a ``device.Batch``) run one persistent
-launch whose CTAs take work items from a queue; how fast they go depends on the workload: how many
-facets a warp applies to a stripe before moving on (facets per pack: inputs re-read per pack
-against the L2 working set of the pack's grids and CF tables), how many stripes one queue item
-holds (queue traffic against load balance) and whether the gridder's warps sum a stripe into a
-shared-memory tile before adding it to the grid (fewer grid additions against shared-memory round
-trips; pays when a stripe's footprints overlap a lot).  ``tune`` times every candidate on a sample
+launch; how fast they go depends on the workload: how many facets a warp applies to a stripe before
+moving on (facets per pack: inputs re-read per pack against the L2 working set of the pack's grids
+and CF tables) and how many stripes a CTA's chunk holds (L1 reuse between its warps against load
+balance).  ``tune`` times every candidate on a sample
 of the workload's blocks (scratch grids and a scratch copy of the visibilities, so the caller's
 data are untouched), keeps the fastest for each call, and caches the choice in a JSON file keyed
 by the workload's shape and the GPU's name.
@@ -23,9 +21,8 @@ import torch
 
 from . import device as D
 
-GRID_CANDIDATES: List[dict] = [dict(facets_per_pack=p, stripes_per_item=s, tiles=t)
-                               for p in (8, 16, 32) for s in (0, 64) for t in (False, True)]
-DEGRID_CANDIDATES: List[dict] = [dict(facets_per_pack=p, stripes_per_item=s) for p in (16, 32, 0) for s in (0, 64)]
+GRID_CANDIDATES: List[dict] = [dict(facets_per_pack=p, stripes_per_item=s) for p in (8, 16, 32) for s in (0, 16)]
+DEGRID_CANDIDATES: List[dict] = [dict(facets_per_pack=p, stripes_per_item=s) for p in (16, 32, 0) for s in (0, 16)]
 
 
 def _cache_path() -> str:
@@ -143,10 +140,7 @@ def tune(vs: D.VisData, facets_grid: Sequence[D.FacetGrid], facets_model: Sequen
                for f in facets_grid]
     table: Dict[str, list] = {"grid": [], "degrid": []}
     best_g, best_gms = None, float("inf")
-    cands = list(grid_candidates or GRID_CANDIDATES)
-    if not vs.single_vis_blocks:  # warp tiles serve single-visibility maps only; the library ignores them otherwise
-        cands = [c for c in cands if not c.get("tiles")]
-    for cand in cands:
+    for cand in (grid_candidates or GRID_CANDIDATES):
         b = D.Batch.create(dev, **cand)
         ms = _time(lambda: D.grid(sv, scratch, pol, jones, batch=b))
         table["grid"].append((cand, round(ms, 3)))

@@ -296,7 +296,7 @@ extern "C" int ddfg_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_po
 }
 
 extern "C" size_t ddfg_batch_workspace_size(void) {
-  return sizeof(unsigned long long) * (size_t)(kGridCounters + kDegridCounters);
+  return sizeof(unsigned int) * (size_t)(kGridCounters + kDegridCounters);
 }
 
 namespace {
@@ -356,8 +356,7 @@ extern "C" int ddfg_degrid_adjoint(const ddfg_vis *vs, const ddfg_jones *js, con
   int rc = degrid_checks(vs, js, pol, facets, nfacets, &policy);
   if (rc) return rc;
   if (nfacets == 0 || vs->nblocks == 0) return DDFG_OK;
-  return ddfg_launch_degrid_adjoint(vs, js, facets, nfacets, policy, pol->npol, ddfg_num_ctas(4),
-                                    (cudaStream_t)stream);
+  return ddfg_launch_degrid_adjoint(vs, js, facets, nfacets, policy, pol->npol, (cudaStream_t)stream);
 }
 
 extern "C" int ddfg_degrid_jones_grad(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_pol *pol,

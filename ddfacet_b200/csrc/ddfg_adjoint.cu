@@ -21,6 +21,8 @@
 #include "ddfg_degridblock.cuh"
 #include "ddfg_gridblock.cuh"
 #include "ddfg_internal.h"
+#include "ddfg_queue.cuh"
+#include "ddfg_single.cuh"
 #include "ddfg_taps.cuh"
 
 namespace ddfg {
@@ -137,7 +139,7 @@ template <int NPOL, int SLOTS>
 __global__ void __launch_bounds__(256) degrid_adjoint_block_kernel(const ddfg_vis vs, const ddfg_jones js,
                                                                    const FacetPack pack, int policy) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ddfg_facet *sf = (ddfg_facet *)smem_raw;
+  ddfg_facet *sf = (ddfg_facet *)((ScatterSmem<NPOL, SLOTS> *)smem_raw + (blockDim.x >> 5));
   double *s_n0m1 = (double *)(sf + DDFG_FACETS_PER_LAUNCH);
   stage_facets(pack, sf);
   __syncthreads();
@@ -150,8 +152,8 @@ __global__ void __launch_bounds__(256) degrid_adjoint_block_kernel(const ddfg_vi
   const int warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   const int64_t nstripes = (vs.nblocks + 31) / 32;
-  LaneTaps<SLOTS> lt;
-  lt.reset();
+  ScatterSmem<NPOL, SLOTS> &ws = ((ScatterSmem<NPOL, SLOTS> *)smem_raw)[warp];
+  ws.clear(lane);
   for (int64_t s = (int64_t)blockIdx.x * nwarps + warp; s < nstripes; s += (int64_t)gridDim.x * nwarps) {
     const int64_t b = s * 32 + lane;
     const bool inrange = b < vs.nblocks;
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(256) degrid_adjoint_block_kernel(const ddfg_vi
       GridRecord<NPOL> rec;
       rec.valid = false;
       if (inrange) adjoint_block_record<NPOL>(d, vs, js, f, policy, s_n0m1[fi], rec);
-      scatter_records<NPOL, SLOTS, true>(rec, f, min(NPOL, f.npol), lt, lane);
+      scatter<NPOL, SLOTS, true>(rec, f, min(NPOL, f.npol), ws, lane);
     }
   }
 }
@@ -171,7 +173,7 @@ template <int NPOL, int SLOTS>
 __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const ddfg_vis vs, const ddfg_jones js,
                                                              const FacetPack pack, int policy) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ddfg_facet *sf = (ddfg_facet *)smem_raw;
+  ddfg_facet *sf = (ddfg_facet *)((ScatterSmem<NPOL, SLOTS> *)smem_raw + (blockDim.x >> 5));
   double *s_n0m1 = (double *)(sf + DDFG_FACETS_PER_LAUNCH);
   stage_facets(pack, sf);
   __syncthreads();
@@ -184,8 +186,8 @@ __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const ddfg_vis vs, 
   const int warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   const int64_t nstripes = (vs.nblocks + 31) / 32;
-  LaneTaps<SLOTS> lt;
-  lt.reset();
+  ScatterSmem<NPOL, SLOTS> &ws = ((ScatterSmem<NPOL, SLOTS> *)smem_raw)[warp];
+  ws.clear(lane);
   for (int64_t s = (int64_t)blockIdx.x * nwarps + warp; s < nstripes; s += (int64_t)gridDim.x * nwarps) {
     const int64_t b = s * 32 + lane;
     DSingleIn in;
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const ddfg_vis vs, 
       const ddfg_facet &f = sf[fi];
       GridRecord<NPOL> rec;
       adjoint_record<NPOL>(in, vs, js, f, policy, s_n0m1[fi], rec);
-      scatter_records<NPOL, SLOTS, true>(rec, f, min(NPOL, f.npol), lt, lane);
+      scatter<NPOL, SLOTS, true>(rec, f, min(NPOL, f.npol), ws, lane);
     }
   }
 }
@@ -367,7 +369,6 @@ __global__ void __launch_bounds__(256) jones_grad_kernel(const ddfg_vis vs, cons
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ddfg_facet *sf = (ddfg_facet *)smem_raw;
   double *s_n0m1 = (double *)(sf + DDFG_FACETS_PER_LAUNCH);
-  float2 *partial = (float2 *)(s_n0m1 + DDFG_FACETS_PER_LAUNCH);
   stage_facets(pack, sf);
   __syncthreads();
   if (threadIdx.x < pack.n) {
@@ -379,9 +380,8 @@ __global__ void __launch_bounds__(256) jones_grad_kernel(const ddfg_vis vs, cons
   const int warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   const int64_t nstripes = (vs.nblocks + 31) / 32;
-  float2 *wpart = partial + warp * 32 * 32;
-  LaneTaps<SLOTS> lt;
-  lt.reset();
+  __shared__ GatherSmem<NPOL> s_gather[8];
+  GatherSmem<NPOL> &ws = s_gather[warp];
   const float2 *J = (const float2 *)js.kms;
   const float kfac = kms_interp_factor(js);
   for (int64_t s = (int64_t)blockIdx.x * nwarps + warp; s < nstripes; s += (int64_t)gridDim.x * nwarps) {
@@ -396,10 +396,8 @@ __global__ void __launch_bounds__(256) jones_grad_kernel(const ddfg_vis vs, cons
       const ddfg_facet &f = sf[fi];
       BlockGeom geo;
       const bool valid = degrid_single_geom_in(in, f, geo);
-      TapJob job;
-      if (valid) job = tap_job(geo, in.gridchan, f);
       float2 mine[NPOL];
-      gather_records<NPOL, SLOTS>(valid, job, f, lt, wpart, lane, mine);
+      gather<NPOL, SLOTS>(valid, geo, in.gridchan, f, ws, lane, mine);
       size_t o0 = 0, o1 = 0;
       M2 d0 = m2_zero(), d1 = m2_zero();
       if (valid) {
@@ -435,7 +433,6 @@ __global__ void __launch_bounds__(256) jones_grad_block_kernel(const ddfg_vis vs
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ddfg_facet *sf = (ddfg_facet *)smem_raw;
   double *s_n0m1 = (double *)(sf + DDFG_FACETS_PER_LAUNCH);
-  float2 *partial = (float2 *)(s_n0m1 + DDFG_FACETS_PER_LAUNCH);
   stage_facets(pack, sf);
   __syncthreads();
   if (threadIdx.x < pack.n) {
@@ -447,9 +444,8 @@ __global__ void __launch_bounds__(256) jones_grad_block_kernel(const ddfg_vis vs
   const int warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   const int64_t nstripes = (vs.nblocks + 31) / 32;
-  float2 *wpart = partial + warp * 32 * 32;
-  LaneTaps<SLOTS> lt;
-  lt.reset();
+  __shared__ GatherSmem<NPOL> s_gather[8];
+  GatherSmem<NPOL> &ws = s_gather[warp];
   const float2 *J = (const float2 *)js.kms;
   const float kfac = kms_interp_factor(js);
   for (int64_t s = (int64_t)blockIdx.x * nwarps + warp; s < nstripes; s += (int64_t)gridDim.x * nwarps) {
@@ -461,10 +457,8 @@ __global__ void __launch_bounds__(256) jones_grad_block_kernel(const ddfg_vis vs
       const ddfg_facet &f = sf[fi];
       BlockGeom geo;
       const bool valid = inrange && degrid_block_geom(vs, f, d, geo);
-      TapJob job;
-      if (valid) job = tap_job(geo, d.gridchan, f);
       float2 mine[NPOL];
-      gather_records<NPOL, SLOTS>(valid, job, f, lt, wpart, lane, mine);
+      gather<NPOL, SLOTS>(valid, geo, d.gridchan, f, ws, lane, mine);
       // the lane's pending sums for one pair of Jones cells (o0, o1): visibilities of a row share
       // them, so the lane adds once per run and the warp combines the last runs
       size_t o0 = 0, o1 = 0;
@@ -537,41 +531,249 @@ __global__ void __launch_bounds__(256) jones_grad_block_kernel(const ddfg_vis vs
   }
 }
 
+// ----------------------------------------------------------------------------------------
+// Stokes I of single visibilities, without smearing and with Jones terms as stored
+// ----------------------------------------------------------------------------------------
+// Both passes see the two Jones matrices through one product a row (ddfg_single.cuh):
+//   * the adjoint value L^H(conj(ph) J0^H g J1) = conj(ph) tr(g J1 J0^H);
+//   * with t = ph s (s the model sample, L(s) = s 1) the Jones gradients are conj(t) g J1 and
+//     t g^H J0, so a row's visibilities need only A = sum conj(t) g: then A J1 and A^H J0.  A warp
+//     sums A a facet in shared memory for as long as its stripes stay on one pair of Jones cells.
+
+template <int SLOTS>
+__global__ void __launch_bounds__(256, 2) adjoint_single_i(const ddfg_vis vs, const ddfg_jones js,
+                                                           const __grid_constant__ FacetTable tab, const Sched sc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using Smem = ScatterSmem<1, SLOTS>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  Smem &ws = ((Smem *)smem_raw)[warp];
+  JonesProduct<true> *keep = (JonesProduct<true> *)((Smem *)smem_raw + nwarps) + warp * sc.max_pack;
+  FacetI *sfi = (FacetI *)((JonesProduct<true> *)((Smem *)smem_raw + nwarps) + nwarps * sc.max_pack);
+  ddfg_facet *sf = (ddfg_facet *)(sfi + sc.max_pack);
+  __shared__ unsigned int ticket;
+  if (threadIdx.x == 0) ticket = 0;
+  ws.clear(lane);
+  const int npk = stage_pack_i(tab, sc, js, 0, sf, sfi);
+  __syncthreads();
+  JonesUse ju;
+  ju.forget();
+  WarpWork work;
+  work.start(sc);
+  for (Work w; work.next(sc, 0, &ticket, lane, w);) {
+    for (long long s = w.s0; s < w.s1; ++s) {
+      const int64_t b = s * 32 + lane;
+      DSingleIn in;
+      in.valid = false;
+      JonesAt at;
+      at.o0 = at.o1 = 0;
+      if (b < vs.nblocks) degrid_load_single<false>(vs, js, b, in);
+      M2 g = m2_zero();
+      if (in.valid) {
+        g = load_corr_matrix(vs, in.irow, in.ch);
+        if (js.mode != 0) at = jones_at(js, in.irow, in.ch);
+      }
+      const unsigned all = __ballot_sync(0xffffffffu, in.valid);
+      if (!all) continue;
+      const int use = ju.stripe(js, in.valid, all, at);
+      for (int fi = 0; fi < npk; ++fi) {
+        const FacetI &f = sfi[fi];
+        float2 t = cadd(g.v[0], g.v[3]);
+        if (use) {
+          const JonesProduct<true> jp = jones_for<true>(js, use, ju, in.valid, at, f.jones_dir, keep + fi, lane);
+          t = cadd(jp.first(g), jp.second(g));
+        }
+        GridRecord<1> rec;
+        rec.valid = in.valid && in.gridchan < f.nband &&
+                    geometry_i(f, dadd(in.U, dmul(in.W, f.cu)), dadd(in.V, dmul(in.W, f.cv)), in.W, in.recip, rec.g);
+        rec.stokes[0] = cmul(t, phasor_turns(-in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * f.n0m1) * kInvC));
+        rec.gridchan = in.gridchan;
+        scatter<1, SLOTS, true>(rec, sf[fi], 1, ws, lane);
+      }
+    }
+  }
+}
+
+// The eight sums over the warp of v[0..7]: lanes 4 j get sum j.
+__device__ __forceinline__ float warp_sum8(const float *v, int lane) {
+  float a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const bool hi = lane & 16;
+    a[i] = (hi ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, hi ? v[i] : v[i + 4], 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const bool hi = lane & 8;
+    b[i] = (hi ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, hi ? a[i] : a[i + 2], 8);
+  }
+  const bool hi = lane & 4;
+  float c = (hi ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, hi ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  return c + __shfl_xor_sync(0xffffffffu, c, 1);
+}
+
+// grad at the two matrices += A J1, A^H J0.
+__device__ __forceinline__ void add_jones_grad_i(const ddfg_jones &js, float2 *grad, int64_t o0, int64_t o1,
+                                                 const M2 &A) {
+  red_add_m2(grad + o0, m2_times(A, load_jones(js, o1)));
+  red_add_m2(grad + o1, m2_times(m2_herm(A), load_jones(js, o0)));
+}
+
+template <int SLOTS>
+__global__ void __launch_bounds__(256, 2) jones_grad_single_i(const ddfg_vis vs, const ddfg_jones js,
+                                                              const __grid_constant__ FacetTable tab, const Sched sc,
+                                                              float2 *grad) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  GatherSmem<1> &ws = ((GatherSmem<1> *)smem_raw)[warp];
+  M2 *sum = (M2 *)((GatherSmem<1> *)smem_raw + nwarps) + warp * sc.max_pack;  // A of the warp's row, a facet
+  FacetI *sfi = (FacetI *)((M2 *)((GatherSmem<1> *)smem_raw + nwarps) + nwarps * sc.max_pack);
+  ddfg_facet *sf = (ddfg_facet *)(sfi + sc.max_pack);
+  __shared__ unsigned int ticket;
+  if (threadIdx.x == 0) ticket = 0;
+  const int npk = stage_pack_i(tab, sc, js, 0, sf, sfi);
+  for (int i = lane; i < npk; i += 32) sum[i] = m2_zero();
+  __syncthreads();
+  JonesUse ju;
+  ju.forget();
+  auto flush = [&](int64_t o0, int64_t o1) {  // a facet a lane
+    __syncwarp();
+    for (int i = lane; i < npk; i += 32) {
+      if (o0 >= 0) add_jones_grad_i(js, grad, o0 + sfi[i].jones_dir, o1 + sfi[i].jones_dir, sum[i]);
+      sum[i] = m2_zero();
+    }
+    __syncwarp();
+  };
+  WarpWork work;
+  work.start(sc);
+  for (Work w; work.next(sc, 0, &ticket, lane, w);) {
+    for (long long s = w.s0; s < w.s1; ++s) {
+      const int64_t b = s * 32 + lane;
+      DSingleIn in;
+      in.valid = false;
+      JonesAt at;
+      at.o0 = at.o1 = 0;
+      if (b < vs.nblocks) degrid_load_single<false>(vs, js, b, in);
+      M2 g = m2_zero();
+      if (in.valid) {
+        g = load_corr_matrix(vs, in.irow, in.ch);
+        at = jones_at(js, in.irow, in.ch);
+      }
+      const unsigned all = __ballot_sync(0xffffffffu, in.valid);
+      if (!all) continue;
+      const int64_t p0 = ju.o0, p1 = ju.o1;
+      const int use = ju.stripe(js, in.valid, all, at);
+      if (use == 2) flush(p0, p1);
+      for (int fi = 0; fi < npk; ++fi) {
+        const FacetI &f = sfi[fi];
+        BlockGeom geo;
+        const bool valid = in.valid && in.gridchan < f.nband &&
+                           geometry_i(f, dadd(in.U, dmul(in.W, f.cu)), dadd(in.V, dmul(in.W, f.cv)), in.W, in.recip, geo);
+        float2 t;
+        gather<1, SLOTS>(valid, geo, in.gridchan, sf[fi], ws, lane, &t);
+        t = valid ? cmul(t, phasor_turns(in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * f.n0m1) * kInvC)) : czero();
+        M2 A;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) A.v[p] = cmul(cconj(t), g.v[p]);
+        if (use == 1) {
+          if (valid) add_jones_grad_i(js, grad, at.o0 + f.jones_dir, at.o1 + f.jones_dir, A);
+        } else {
+          const float v = warp_sum8((const float *)A.v, lane);
+          if ((lane & 3) == 0) ((float *)&sum[fi])[lane >> 2] += v;
+        }
+      }
+    }
+  }
+  flush(ju.o0, ju.o1);
+}
+
 }  // namespace ddfg
 
 using namespace ddfg;
 
+namespace {
+
+// Whether the kernels for Stokes I take the call.
+bool adjoint_is_i(const ddfg_vis *vs, const ddfg_jones *js, int policy) {
+  return vs->single_vis_blocks && policy == D_DIAG_FROM_I && !vs->uvw_dt && jones_as_stored(js);
+}
+
+// One launch over facets[0..n), n <= 16: the adjoint (grad NULL) or the Jones gradient.
+template <int SL>
+int launch_i(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet *facets, int n, float2 *grad,
+             cudaStream_t stream) {
+  FacetTable tab;
+  for (int i = 0; i < n; ++i) tab.f[i] = facets[i];
+  Sched sc{};
+  sc.nfacets = sc.max_pack = n;
+  sc.npacks = 1;
+  sc.nstripes = (vs->nblocks + 31) / 32;
+  const size_t smem = (sizeof(ddfg_facet) + sizeof(FacetI)) * (size_t)n +
+                      8 * (grad ? sizeof(GatherSmem<1>) + n * sizeof(M2)
+                                : sizeof(ScatterSmem<1, SL>) + n * sizeof(JonesProduct<true>));
+  const void *kern = grad ? (const void *)jones_grad_single_i<SL> : (const void *)adjoint_single_i<SL>;
+  int per_sm = 0;
+  const int rc = ddfg_kernel_prepare(kern, 256, smem, &per_sm);
+  if (rc) return rc;
+  const int ctas = ddfg_num_ctas(per_sm);
+  sched_split(sc, nullptr, ctas, 8);
+  if (grad) jones_grad_single_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, sc, grad);
+  else adjoint_single_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, sc);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "degrid backward launch: %s", cudaGetErrorString(e));
+  return DDFG_OK;
+}
+
+template <int NP, int SL>
+int launch_adjoint(const ddfg_vis *vs, const ddfg_jones *js, const FacetPack &pack, int policy, cudaStream_t stream) {
+  const size_t smem = 8 * sizeof(ScatterSmem<NP, SL>) + (sizeof(ddfg_facet) + sizeof(double)) * DDFG_FACETS_PER_LAUNCH;
+  const void *kern = vs->single_vis_blocks ? (const void *)degrid_adjoint_kernel<NP, SL>
+                                           : (const void *)degrid_adjoint_block_kernel<NP, SL>;
+  int per_sm = 0;
+  const int rc = ddfg_kernel_prepare(kern, 256, smem, &per_sm);
+  if (rc) return rc;
+  const int ctas = ddfg_num_ctas(per_sm);
+  if (vs->single_vis_blocks) degrid_adjoint_kernel<NP, SL><<<ctas, 256, smem, stream>>>(*vs, *js, pack, policy);
+  else degrid_adjoint_block_kernel<NP, SL><<<ctas, 256, smem, stream>>>(*vs, *js, pack, policy);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "degrid_adjoint launch: %s", cudaGetErrorString(e));
+  return DDFG_OK;
+}
+}  // namespace
+
 int ddfg_launch_degrid_adjoint(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet *facets, int nfacets,
-                               int policy, int nvispol, int num_ctas, cudaStream_t stream) {
+                               int policy, int nvispol, cudaStream_t stream) {
   int max_support = 1;
   for (int i = 0; i < nfacets; ++i) max_support = max(max_support, facets[i].max_support);
-  const int slots = tap_slots(max_support);
-  const size_t smem = sizeof(ddfg_facet) * DDFG_FACETS_PER_LAUNCH + sizeof(double) * DDFG_FACETS_PER_LAUNCH;
+  const int slots = tap_slots(max_support, nvispol);
   const int npacks = (nfacets + DDFG_FACETS_PER_LAUNCH - 1) / DDFG_FACETS_PER_LAUNCH;  // balanced packs
   for (int ip = 0; ip < npacks; ++ip) {
     const int f0 = (int)(((long long)ip * nfacets) / npacks);
     FacetPack pack;
     pack.n = (int)(((long long)(ip + 1) * nfacets) / npacks) - f0;
+    if (adjoint_is_i(vs, js, policy)) {
+      const int rc = slots == 2 ? launch_i<2>(vs, js, facets + f0, pack.n, nullptr, stream)
+                                : launch_i<4>(vs, js, facets + f0, pack.n, nullptr, stream);
+      if (rc) return rc;
+      continue;
+    }
     for (int i = 0; i < pack.n; ++i) pack.f[i] = facets[f0 + i];
-#define LAUNCH_A(NP, SL)                                                                      \
-  do {                                                                                        \
-    if (vs->single_vis_blocks)                                                                \
-      degrid_adjoint_kernel<NP, SL><<<num_ctas, 256, smem, stream>>>(*vs, *js, pack, policy);       \
-    else                                                                                      \
-      degrid_adjoint_block_kernel<NP, SL><<<num_ctas, 256, smem, stream>>>(*vs, *js, pack, policy); \
-  } while (0)
-#define LAUNCH_A_NP(SL)              \
-  switch (nvispol) {                 \
-    case 1: LAUNCH_A(1, SL); break;  \
-    case 2: LAUNCH_A(2, SL); break;  \
-    case 3: LAUNCH_A(3, SL); break;  \
-    default: LAUNCH_A(4, SL); break; \
-  }
-    if (slots == 2) { LAUNCH_A_NP(2) } else if (slots == 4) { LAUNCH_A_NP(4) } else { LAUNCH_A_NP(8) }
-#undef LAUNCH_A_NP
+    int rc;
+#define LAUNCH_A(NP, SL) rc = launch_adjoint<NP, SL>(vs, js, pack, policy, stream)
+    if (slots == 2) {
+      switch (nvispol) {
+        case 1: LAUNCH_A(1, 2); break;
+        case 2: LAUNCH_A(2, 2); break;
+        case 3: LAUNCH_A(3, 2); break;
+        default: LAUNCH_A(4, 2); break;
+      }
+    } else if (nvispol == 1) {
+      LAUNCH_A(1, 4);
+    } else {
+      LAUNCH_A(2, 4);
+    }
 #undef LAUNCH_A
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "degrid_adjoint launch: %s", cudaGetErrorString(e));
+    if (rc) return rc;
   }
   return DDFG_OK;
 }
@@ -580,9 +782,8 @@ int ddfg_launch_jones_grad(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_
                            int policy, int nvispol, void *grad, int num_ctas, cudaStream_t stream) {
   int max_support = 1;
   for (int i = 0; i < nfacets; ++i) max_support = max(max_support, facets[i].max_support);
-  const int slots = tap_slots(max_support);
-  const size_t smem = sizeof(ddfg_facet) * DDFG_FACETS_PER_LAUNCH + sizeof(double) * DDFG_FACETS_PER_LAUNCH +
-                      (nvispol == 1 ? 8 * kPartialBytesPerWarp : 0);
+  const int slots = tap_slots(max_support, nvispol);
+  const size_t smem = sizeof(ddfg_facet) * DDFG_FACETS_PER_LAUNCH + sizeof(double) * DDFG_FACETS_PER_LAUNCH;
   float2 *g = (float2 *)grad;
   int per_sm = 0;
   const int npacks = (nfacets + DDFG_FACETS_PER_LAUNCH - 1) / DDFG_FACETS_PER_LAUNCH;  // balanced packs
@@ -590,6 +791,12 @@ int ddfg_launch_jones_grad(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_
     const int f0 = (int)(((long long)ip * nfacets) / npacks);
     FacetPackD pack;
     pack.n = (int)(((long long)(ip + 1) * nfacets) / npacks) - f0;
+    if (adjoint_is_i(vs, js, policy)) {
+      const int rc = slots == 2 ? launch_i<2>(vs, js, facets + f0, pack.n, g, stream)
+                                : launch_i<4>(vs, js, facets + f0, pack.n, g, stream);
+      if (rc) return rc;
+      continue;
+    }
     for (int i = 0; i < pack.n; ++i) pack.f[i] = facets[f0 + i];
 #define LAUNCH_J(NP, SL)                                                                                   \
   do {                                                                                                     \
@@ -601,15 +808,18 @@ int ddfg_launch_jones_grad(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_
       jones_grad_block_kernel<NP, SL><<<num_ctas, 256, smem, stream>>>(*vs, *js, pack, policy, g);           \
     }                                                                                                      \
   } while (0)
-#define LAUNCH_J_NP(SL)              \
-  switch (nvispol) {                 \
-    case 1: LAUNCH_J(1, SL); break;  \
-    case 2: LAUNCH_J(2, SL); break;  \
-    case 3: LAUNCH_J(3, SL); break;  \
-    default: LAUNCH_J(4, SL); break; \
-  }
-    if (slots == 2) { LAUNCH_J_NP(2) } else if (slots == 4) { LAUNCH_J_NP(4) } else { LAUNCH_J_NP(8) }
-#undef LAUNCH_J_NP
+    if (slots == 2) {
+      switch (nvispol) {
+        case 1: LAUNCH_J(1, 2); break;
+        case 2: LAUNCH_J(2, 2); break;
+        case 3: LAUNCH_J(3, 2); break;
+        default: LAUNCH_J(4, 2); break;
+      }
+    } else if (nvispol == 1) {
+      LAUNCH_J(1, 4);
+    } else {
+      LAUNCH_J(2, 4);
+    }
 #undef LAUNCH_J
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "jones_grad launch: %s", cudaGetErrorString(e));

@@ -36,11 +36,25 @@ __device__ __forceinline__ float cabs2(float2 a) { return sqrtf(a.x * a.x + a.y 
 __device__ __forceinline__ float2 cmuli(float2 a) { return make_float2(-a.y, a.x); }  // a * i
 __device__ __forceinline__ float2 czero() { return make_float2(0.f, 0.f); }
 
+// acc + x y, and acc + conj(x) y, four FMAs.
+__device__ __forceinline__ float2 cfma(float2 x, float2 y, float2 acc) {
+  return make_float2(fmaf(-x.y, y.y, fmaf(x.x, y.x, acc.x)), fmaf(x.y, y.x, fmaf(x.x, y.y, acc.y)));
+}
+__device__ __forceinline__ float2 cfma_conj(float2 x, float2 y, float2 acc) {
+  return make_float2(fmaf(x.y, y.y, fmaf(x.x, y.x, acc.x)), fmaf(-x.y, y.x, fmaf(x.x, y.y, acc.y)));
+}
+
 // grid[cell] += v as one vector reduction without a return value (red.global.add.v2.f32,
 // sm_90+): the same addition as atomicAdd(float2*), which is issued as a returning atomic, but
 // the issuing warp does not wait for the L2 round trip.
 __device__ __forceinline__ void red_add(float2 *p, float2 v) {
   asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
+}
+
+// *p += v in global memory (atomicAdd through a pointer of unknown space also compiles the
+// shared-memory loop).
+__device__ __forceinline__ void red_add_double(double *p, double v) {
+  asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
 // 2x2 complex matrix, element order [0]=(0,0) [1]=(0,1) [2]=(1,0) [3]=(1,1) (JonesServer.h:38-81)
@@ -153,6 +167,14 @@ __device__ __forceinline__ void norm_jones(M2 &j, const ddfg_jones &js, double u
   }
 }
 
+// The Jones weight BB of a visibility (JonesServer.cc:290-297).  Its roundings are spelled out: the
+// FP64 Jones sums add it up, and every kernel that forms it has to give the same number.
+__device__ __forceinline__ float jones_weight(const M2 &j0, const M2 &j1) {
+  auto mag = [](float2 a) { return __fsqrt_rn(__fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y))); };
+  const float t = __fmul_rn(__fmaf_rn(mag(j0.v[0]), mag(j1.v[0]), __fmul_rn(mag(j0.v[3]), mag(j1.v[3]))), 0.5f);
+  return __fmul_rn(t, t);
+}
+
 // Cached Jones state of one block walk.  The reference recomputes the beam and DD Jones only
 // when the antennas, the time slot or the Jones channel change; the DD Jones normalisation
 // reads the uvw of the visibility at which that happened, which is kept so the cached and
@@ -215,8 +237,7 @@ struct JonesCache {
       }
       j0 = a;
       j1 = b;
-      const float t = (cabs2(j0.v[0]) * cabs2(j1.v[0]) + cabs2(j0.v[3]) * cabs2(j1.v[3])) * 0.5f;
-      bb = t * t;
+      bb = jones_weight(j0, j1);
     }
     return changed;
   }
@@ -262,14 +283,7 @@ __device__ __forceinline__ void jones_pair_at(const ddfg_jones &js, int idir_kms
   }
   j0 = a;
   j1 = b;
-  const float t = (cabs2(a.v[0]) * cabs2(b.v[0]) + cabs2(a.v[3]) * cabs2(b.v[3])) * 0.5f;
-  bb = t * t;
-}
-
-// The same, loading the indices of row irow and channel ichan.
-__device__ __forceinline__ void jones_pair(const ddfg_jones &js, int idir_kms, int idir_beam, int64_t irow, int ichan,
-                                           double u, double v, M2 &j0, M2 &j1, float &bb) {
-  jones_pair_at(js, idir_kms, idir_beam, jones_idx(js, irow, ichan), u, v, j0, j1, bb);
+  bb = jones_weight(a, b);
 }
 
 // ----------------------------------------------------------------------------------------
@@ -385,60 +399,7 @@ struct BlockGeom {
   int locx, locy;  // centre cell
   int sup;         // (S-1)/2
   int S;           // support
-  unsigned inv;    // ceil(65536 / S): t / S == (t * inv) >> 16 for every tap t < S*S (S <= 63)
-  const float2 *cf;  // first tap of the [io][jo] sub-kernel (S*S taps, row-major sy, sx)
-  int cfoff;       // the same tap as an element offset from cf_data
-};
-
-// Footprint of a block packed for a warp broadcast: cell index of the footprint's first tap in
-// the facet grid array, CF element offset, and support with its reciprocal.
-struct TapJob {
-  int base;        // ((band * npol) * ny + locy - sup) * nx + locx - sup
-  int cfoff;
-  int s_inv;       // S | inv << 8
-};
-__device__ __forceinline__ TapJob tap_job(const BlockGeom &g, int band, const ddfg_facet &f) {
-  TapJob j;
-  j.base = ((band * f.npol) * f.ny + g.locy - g.sup) * f.nx + g.locx - g.sup;
-  j.cfoff = g.cfoff;
-  j.s_inv = g.S | (int)(g.inv << 8);
-  return j;
-}
-__device__ __forceinline__ TapJob shfl_job(const TapJob &j, int src) {
-  TapJob o;
-  o.base = __shfl_sync(0xffffffffu, j.base, src);
-  o.cfoff = __shfl_sync(0xffffffffu, j.cfoff, src);
-  o.s_inv = __shfl_sync(0xffffffffu, j.s_inv, src);
-  return o;
-}
-
-// Register slots per lane that hold a footprint of the given support (S*S taps over 32 lanes).
-inline int tap_slots(int max_support) {
-  const int t = max_support * max_support;
-  return t <= 64 ? 2 : (t <= 128 ? 4 : 8);
-}
-
-// Per-lane tap offsets for the current support and grid width, recomputed when either changes:
-// lane l owns taps t = l + 32 k (k < SLOTS), at cell offset (t / S) * nx + t % S.
-template <int SLOTS>
-struct LaneTaps {
-  int S, NX;
-  int off[SLOTS];
-  __device__ __forceinline__ void reset() { S = -1; NX = -1; }
-  // The offsets depend on the grid width too: facets of one launch may differ in size.
-  __device__ __forceinline__ void set(int s_inv, int nx, int lane) {
-    const int s = s_inv & 255;
-    if (s == S && nx == NX) return;
-    S = s;
-    NX = nx;
-    const unsigned inv = (unsigned)s_inv >> 8;
-#pragma unroll
-    for (int k = 0; k < SLOTS; ++k) {
-      const int t = lane + 32 * k;
-      const int sy = (int)(((unsigned)t * inv) >> 16);
-      off[k] = (t < s * s) ? sy * nx + (t - sy * s) : -1;
-    }
-  }
+  int cfoff;       // first tap of the [io][jo] sub-kernel (S*S taps, row-major sy, sx) from cf_data
 };
 
 // dbg (nullable, [7]): the intermediate integers {iw, plane, locx, locy, offx, offy, k} as far as
@@ -455,7 +416,7 @@ __device__ __forceinline__ bool block_geometry(const ddfg_facet &f, double umean
   if (iw < 0) return false;
   const int plane = (wmean > 0.) ? (int)iw : f.nw + (int)iw;
   if (dbg) dbg[1] = plane;
-  const int S = f.cf_support[plane];
+  const int S = __ldg(f.cf_support + plane);
   const int O = f.overs;
   const int nconv = S * O;
   const int sup = (S - 1) / 2;  // (nConvX/OverS-1)/2
@@ -487,9 +448,7 @@ __device__ __forceinline__ bool block_geometry(const ddfg_facet &f, double umean
   g.locy = (int)ly;
   g.sup = sup;
   g.S = S;
-  g.inv = (65536u + (unsigned)S - 1u) / (unsigned)S;
-  g.cfoff = (int)(f.cf_offset[plane] + (int64_t)k * S * S);
-  g.cf = (const float2 *)f.cf_data + g.cfoff;
+  g.cfoff = (int)(__ldg(f.cf_offset + plane) + (int64_t)k * S * S);
   return true;
 }
 

@@ -1,4 +1,4 @@
-// The degridder's per-block steps (shared by the direct and the tile-sorted kernels):
+// The degridder's per-block steps:
 // block means and footprint (degridder.h:138-200) and the per-visibility correction and
 // subtraction (degridder.h:214-264).
 #pragma once
@@ -37,26 +37,36 @@ __device__ __forceinline__ void degrid_block_header(const ddfg_vis &vs, int64_t 
   d.freqmean = (nc == 1) ? fm : fm / (double)nc;
 }
 
+// The unweighted row means of (u + w Cu, v + w Cv, w) and 1 / wavelength of the block's mean frequency.
+struct RowMeans {
+  double u, v, w, recip;
+};
+__device__ __forceinline__ RowMeans degrid_row_means(const ddfg_vis &vs, double cu, double cv, const DegridBlock &d) {
+  RowMeans m;
+  m.u = m.v = m.w = 0.;
+  for (int inx = 0; inx < d.nrows; ++inx) {
+    const double *up = vs.uvw + 3 * (int64_t)d.rows[inx];
+    m.u = dadd(m.u, dadd(up[0], dmul(up[2], cu)));
+    m.v = dadd(m.v, dadd(up[1], dmul(up[2], cv)));
+    m.w = dadd(m.w, up[2]);
+  }
+  if (d.nrows > 1) {
+    const double dn = (double)d.nrows;
+    m.u = m.u / dn;
+    m.v = m.v / dn;
+    m.w = m.w / dn;
+  }
+  m.recip = (d.ch1 - d.ch0 == 1 && vs.recip_wvl) ? vs.recip_wvl[d.ch0] : d.freqmean / kC;
+  return m;
+}
+
 // Footprint of block b on facet f; false when the reference skips it.
 __device__ __forceinline__ bool degrid_block_geom(const ddfg_vis &vs, const ddfg_facet &f, const DegridBlock &d,
                                                   BlockGeom &g, int *dbg = nullptr) {
   if (d.ch1 <= d.ch0 || d.nrows <= 0) return false;
   if (d.gridchan < 0 || d.gridchan >= f.nband) return false;
-  double um = 0., vm = 0., wm = 0.;
-  for (int inx = 0; inx < d.nrows; ++inx) {
-    const double *up = vs.uvw + 3 * (int64_t)d.rows[inx];
-    um = dadd(um, dadd(up[0], dmul(up[2], f.cu)));
-    vm = dadd(vm, dadd(up[1], dmul(up[2], f.cv)));
-    wm = dadd(wm, up[2]);
-  }
-  if (d.nrows > 1) {
-    const double dn = (double)d.nrows;
-    um = um / dn;
-    vm = vm / dn;
-    wm = wm / dn;
-  }
-  const double rw = (d.ch1 - d.ch0 == 1 && vs.recip_wvl) ? vs.recip_wvl[d.ch0] : d.freqmean / kC;
-  return block_geometry(f, um, vm, wm, rw, g, dbg);
+  const RowMeans m = degrid_row_means(vs, f.cu, f.cv, d);
+  return block_geometry(f, m.u, m.v, m.w, m.recip, g, dbg);
 }
 
 // The block's Stokes -> correlation prediction with the per-block Jones (BDAJones), smearing
@@ -164,22 +174,6 @@ __device__ __forceinline__ void degrid_block_apply_warp(const ddfg_vis &vs, cons
   }
 }
 
-// Single-visibility blocks (one row, one channel): degridder.h:138-264 without the loops.
-__device__ __forceinline__ bool degrid_single_geom(const ddfg_vis &vs, const ddfg_facet &f, int64_t b, int &ch,
-                                                   int64_t &irow, int &gridchan, BlockGeom &g) {
-  const int64_t start = vs.block_start[b];
-  ch = vs.bda_map[start];
-  irow = vs.bda_map[start + 2];
-  gridchan = vs.chan_map[ch];
-  if (gridchan < 0 || gridchan >= f.nband) return false;
-  const double *up = vs.uvw + 3 * irow;
-  const double W = up[2];
-  const double um = dadd(up[0], dmul(W, f.cu));
-  const double vm = dadd(up[1], dmul(W, f.cv));
-  const double rw = vs.recip_wvl ? vs.recip_wvl[ch] : vs.freqs[ch] / kC;
-  return block_geometry(f, um, vm, W, rw, g);
-}
-
 // Facet-independent inputs of a single-visibility block for the degridder, loaded once and
 // shared by every facet of a launch.
 struct DSingleIn {
@@ -190,6 +184,8 @@ struct DSingleIn {
   JonesIdx jx;  // valid when js.mode != 0
 };
 
+// JONES: the Jones indices too.
+template <bool JONES = true>
 __device__ __forceinline__ void degrid_load_single(const ddfg_vis &vs, const ddfg_jones &js, int64_t b,
                                                    DSingleIn &in) {
   const int64_t start = vs.block_start[b];
@@ -203,10 +199,10 @@ __device__ __forceinline__ void degrid_load_single(const ddfg_vis &vs, const ddf
   in.W = up[2];
   in.recip = vs.recip_wvl ? vs.recip_wvl[in.ch] : vs.freqs[in.ch] / kC;
   in.nu = vs.freqs[in.ch];
-  if (js.mode != 0) in.jx = jones_idx(js, in.irow, in.ch);
+  if (JONES && js.mode != 0) in.jx = jones_idx(js, in.irow, in.ch);
 }
 
-// degrid_single_geom from preloaded inputs.
+// The footprint from preloaded inputs.
 __device__ __forceinline__ bool degrid_single_geom_in(const DSingleIn &in, const ddfg_facet &f, BlockGeom &g) {
   if (!in.valid || in.gridchan >= f.nband) return false;
   const double um = dadd(in.U, dmul(in.W, f.cu));
@@ -214,7 +210,7 @@ __device__ __forceinline__ bool degrid_single_geom_in(const DSingleIn &in, const
   return block_geometry(f, um, vm, in.W, in.recip, g);
 }
 
-// The prediction of facet f for a single visibility (what degrid_single_apply subtracts):
+// The prediction of facet f for a single visibility (what the degridder subtracts):
 // Stokes -> correlations, J0 M J1^H, phasor exp(+i nu angle) and smearing (degridder.h:214-261).
 template <int NPOL>
 __device__ __forceinline__ M2 degrid_single_pred(const DSingleIn &in, const ddfg_vis &vs, const ddfg_jones &js,
@@ -233,40 +229,6 @@ __device__ __forceinline__ M2 degrid_single_pred(const DSingleIn &in, const ddfg
   const float dec = (float)decorr_factor(vs, f, in.nu, in.irow);
   const float2 ph = cscale(phasor_turns(in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * n0m1) * kInvC), dec);
   return m2_scale(cv, ph);
-}
-
-template <int NPOL>
-__device__ __forceinline__ void degrid_single_apply(const ddfg_vis &vs, const ddfg_jones &js, const ddfg_facet &f,
-                                                    const DegridParams &dp, int ch, int64_t irow, const float2 *pred) {
-  float2 s[4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) s[p] = (p < NPOL) ? pred[p] : czero();
-  M2 cv = corr_from_stokes(dp.policy, s);
-  const double *up = vs.uvw + 3 * irow;
-  const double nu = vs.freqs[ch];
-  if (js.mode != 0) {
-    M2 j0, j1;
-    float bb;
-    jones_pair(js, f.idir_kms, f.idir_beam, irow, ch, up[0], up[1], j0, j1, bb);
-    cv = m2_times(m2_times(j0, cv), m2_herm(j1));
-  }
-  const float dec = (float)decorr_factor(vs, f, nu, irow);
-  const double n0m1 = sqrt(1. - f.l0 * f.l0 - f.m0 * f.m0) - 1.;
-  const float2 ph = cscale(phasor_turns(nu * (up[0] * f.l0 + up[1] * f.m0 + up[2] * n0m1) * kInvC), dec);
-  const M2 vb = m2_scale(cv, ph);
-  float2 *vp = (float2 *)vs.vis + (irow * vs.nchan + ch) * (int64_t)vs.ncorr;
-  if (vs.ncorr == 4) {
-    float4 a = *(float4 *)vp, c = *(float4 *)(vp + 2);
-    a.x -= vb.v[0].x; a.y -= vb.v[0].y; a.z -= vb.v[1].x; a.w -= vb.v[1].y;
-    c.x -= vb.v[2].x; c.y -= vb.v[2].y; c.z -= vb.v[3].x; c.w -= vb.v[3].y;
-    *(float4 *)vp = a;
-    *(float4 *)(vp + 2) = c;
-  } else if (vs.ncorr == 2) {
-    vp[0] = csub(vp[0], vb.v[0]);
-    vp[1] = csub(vp[1], vb.v[3]);
-  } else {
-    vp[0] = csub(vp[0], vb.v[0]);
-  }
 }
 
 }  // namespace ddfg

@@ -1,4 +1,4 @@
-// The gridder's per-block walk (shared by the direct and the tile-sorted gridding kernels).
+// The gridder's per-block walk.
 #pragma once
 #include "ddfg_common.cuh"
 
@@ -28,6 +28,7 @@ struct GridRecord {
   double sumsqw;          // ThisSumSqWeights
   int ch0;                // first channel of the block
   bool single_chan;       // one channel: its channel sums are the block sums
+  float bb;               // the Jones factor of sumjones (single visibilities)
 };
 
 // Facet-independent inputs of a single-visibility block (one row, one channel), loaded once
@@ -41,6 +42,8 @@ struct SingleIn {
   JonesIdx jx;  // valid when js.mode != 0
 };
 
+// JONES: the Jones indices too.
+template <bool JONES = true>
 __device__ __forceinline__ void load_single(const ddfg_vis &vs, const ddfg_jones &js, const GridParams &gp, int64_t b,
                                             SingleIn &in) {
   in.valid = false;
@@ -73,7 +76,7 @@ __device__ __forceinline__ void load_single(const ddfg_vis &vs, const ddfg_jones
       in.vm.v[0] = vp[0]; in.vm.v[1] = czero(); in.vm.v[2] = czero(); in.vm.v[3] = vp[0];
     }
   }
-  if (js.mode != 0) in.jx = jones_idx(js, irow, ch);
+  if (JONES && js.mode != 0) in.jx = jones_idx(js, irow, ch);
   in.valid = true;
 }
 
@@ -102,9 +105,9 @@ __device__ __forceinline__ void grid_single_facet(const SingleIn &in, const ddfg
   const double fw = in.fw;
   const double fwd = fw * dec * dec;
   double sumjones = 0.;
+  float bb = 0.f;
   if (js.mode != 0) {
     M2 j0, j1;
-    float bb;
     // mode 1 normalises with the row's uvw, mode 2 with the block mean (gridder.h:236, 294)
     jones_pair_at(js, f.idir_kms, f.idir_beam, in.jx, js.mode == 1 ? U : umean, js.mode == 1 ? V : vmean, j0, j1,
                   bb);
@@ -132,16 +135,7 @@ __device__ __forceinline__ void grid_single_facet(const SingleIn &in, const ddfg
   rec.sumsqw = fwd;
   rec.ch0 = in.ch;
   rec.single_chan = true;
-}
-
-// A block of exactly one row and one channel (every block of a map built without averaging).
-template <int NPOL>
-__device__ __forceinline__ void grid_single_record(const ddfg_vis &vs, const ddfg_jones &js, const ddfg_facet &f,
-                                                   const GridParams &gp, int64_t b, double n0m1,
-                                                   GridRecord<NPOL> &rec) {
-  SingleIn in;
-  load_single(vs, js, gp, b, in);
-  grid_single_facet<NPOL>(in, vs, js, f, gp, n0m1, rec);
+  rec.bb = bb;
 }
 
 // Walk one block for one facet: gridder.h:184-351.
@@ -320,14 +314,12 @@ __device__ __forceinline__ void grid_block_add_chan_sums(const ddfg_vis &vs, con
   }
 }
 
-// The warp's 32 records' contributions to the weight and Jones sums (gridder.h:363-373): one
-// shared-memory update per warp when every valid lane grids into the same band, per lane
-// otherwise.  Must be called by all 32 lanes.
-template <int NPOL, bool SINGLE = false>
-__device__ __forceinline__ void warp_add_block_sums(const ddfg_vis &vs, const ddfg_jones &js, const ddfg_facet &f,
-                                                    const GridParams &gp, int64_t b, const GridRecord<NPOL> &rec,
-                                                    int npol_used, double *a_sumwt, double *a_sumj, double *a_chan,
-                                                    JonesCache &jc, bool chan_sums_done = false) {
+// The warp's 32 records' contributions to the weight and Jones sums (gridder.h:363-373), added to
+// the warp's own shared copies (a_sumwt, a_sumj): once per warp when every valid lane grids into the
+// same band, per lane otherwise.  Must be called by all 32 lanes.
+template <int NPOL>
+__device__ __forceinline__ void warp_add_sums(const ddfg_jones &js, const ddfg_facet &f, const GridRecord<NPOL> &rec,
+                                              int npol_used, double *a_sumwt, double *a_sumj) {
   const unsigned vmask = __ballot_sync(0xffffffffu, rec.valid);
   if (!vmask) return;
   const int lane = threadIdx.x & 31;
@@ -352,15 +344,66 @@ __device__ __forceinline__ void warp_add_block_sums(const ddfg_vis &vs, const dd
       atomicAdd(&a_sumj[f.nband + g], (double)npol_used * qsum);
     }
   }
-  if (js.mode != 0 && rec.valid && !chan_sums_done) {
-    if (SINGLE) {
-      atomicAdd(&a_chan[rec.ch0], (double)npol_used * rec.sumjones);
-      atomicAdd(&a_chan[vs.nchan + rec.ch0], (double)npol_used * rec.sumsqw);
+}
+
+// The same for averaged blocks, with the per-channel Jones sums into the CTA's shared copy.
+template <int NPOL>
+__device__ __forceinline__ void warp_add_block_sums(const ddfg_vis &vs, const ddfg_jones &js, const ddfg_facet &f,
+                                                    const GridParams &gp, int64_t b, const GridRecord<NPOL> &rec,
+                                                    int npol_used, double *a_sumwt, double *a_sumj, double *a_chan,
+                                                    JonesCache &jc, bool chan_sums_done = false) {
+  warp_add_sums<NPOL>(js, f, rec, npol_used, a_sumwt, a_sumj);
+  if (js.mode != 0 && rec.valid && !chan_sums_done)
+    grid_block_add_chan_sums<NPOL>(vs, js, f, gp, b, rec, (double)npol_used, a_chan, jc);
+}
+
+// The same for single visibilities.  `all` is the lanes with a visibility and wsum their weights'
+// sum, formed once a stripe: a facet that takes them all, in one band and without smearing, needs no
+// reduction of its own for the weights, and none for the Jones sums while their factor is one
+// number (a row's channels share their Jones terms).  s_chan: the CTA's per-channel Jones sums, or
+// NULL (kSharedChannels).
+template <int NPOL>
+__device__ __forceinline__ void warp_add_single_sums(const ddfg_vis &vs, const ddfg_jones &js, const ddfg_facet &f,
+                                                     const GridRecord<NPOL> &rec, int npol_used, unsigned all,
+                                                     bool one_band, double wsum, double *a_sumwt, double *a_sumj,
+                                                     double *s_chan) {
+  const unsigned vmask = __ballot_sync(0xffffffffu, rec.valid);
+  if (!vmask) return;
+  const int lane = threadIdx.x & 31, lead = __ffs(vmask) - 1;
+  const float bb0 = __shfl_sync(0xffffffffu, rec.bb, lead);
+  const bool plain = vmask == all && one_band && !vs.uvw_dt &&
+                     (js.mode == 0 || __all_sync(0xffffffffu, !rec.valid || rec.bb == bb0));
+  if (plain) {
+    if (lane == lead) {
+      const int g = rec.gridchan;
+      for (int p = 0; p < npol_used; ++p) a_sumwt[g * f.npol + p] += wsum;
+      if (js.mode != 0) {
+        a_sumj[g] += (double)npol_used * ((double)bb0 * wsum);
+        a_sumj[f.nband + g] += (double)npol_used * wsum;
+      }
+    }
+    __syncwarp();
+  } else {
+    warp_add_sums<NPOL>(js, f, rec, npol_used, a_sumwt, a_sumj);
+  }
+  if (js.mode != 0 && rec.valid && f.sumjones_chan) {
+    const double j = (double)npol_used * rec.sumjones, q = (double)npol_used * rec.sumsqw;
+    if (s_chan) {
+      atomicAdd(&s_chan[rec.ch0], j);
+      atomicAdd(&s_chan[vs.nchan + rec.ch0], q);
     } else {
-      grid_block_add_chan_sums<NPOL>(vs, js, f, gp, b, rec, (double)npol_used, a_chan, jc);
+      red_add_double(f.sumjones_chan + rec.ch0, j);
+      red_add_double(f.sumjones_chan + vs.nchan + rec.ch0, q);
     }
   }
 }
+
+// Channels up to which the single-visibility gridder keeps the per-channel Jones sums in shared
+// memory.  Straight to global memory, 32 neighbouring channels are 16 sectors a stripe and facet and
+// a shared copy (4 KB a facet at 256 channels) would cost the tile its room; with few channels every
+// warp of the GPU adds to the same few sectors (16 channels, one facet, 340,000 visibilities: 230 us
+// against 60 us with shared copies).
+constexpr int kSharedChannels = 128;
 
 // Visibilities of block b (rows x channels, flagged ones included).
 __device__ __forceinline__ int64_t block_nvis(const ddfg_vis &vs, int64_t b) {
@@ -368,7 +411,7 @@ __device__ __forceinline__ int64_t block_nvis(const ddfg_vis &vs, int64_t b) {
   return (int64_t)(vs.bda_map[2 + b] - 2) * (vs.bda_map[start + 1] - vs.bda_map[start]);
 }
 
-// The FP64 block means of grid_block_record in the reference's order (gridder.h:272-279): one
+// The FP64 sums behind the block means of grid_block_record, in the reference's order (gridder.h:272-279): one
 // lane, only the flags read per visibility.  Keeping this sum sequential keeps every integer index
 // derived from it bit-exact.
 struct BlockMeans {
@@ -376,20 +419,17 @@ struct BlockMeans {
   int nvis, last_ch;
 };
 
-__device__ __forceinline__ BlockMeans grid_block_means(const ddfg_vis &vs, const ddfg_facet &f, int64_t b) {
+__device__ __forceinline__ BlockMeans grid_block_sums(const ddfg_vis &vs, double cu, double cv, const int32_t *rows,
+                                                      int nrows, int ch0, int ch1) {
   BlockMeans m;
   m.u = m.v = m.w = m.nu = 0.;
   m.nvis = 0;
-  const int64_t start = vs.block_start[b];
-  const int nrows_blk = vs.bda_map[2 + b] - 2;
-  const int ch0 = vs.bda_map[start], ch1 = vs.bda_map[start + 1];
   m.last_ch = ch0;
-  const int32_t *rows = vs.bda_map + start + 2;
-  for (int inx = 0; inx < nrows_blk; ++inx) {
+  for (int inx = 0; inx < nrows; ++inx) {
     const int64_t irow = rows[inx];
     const double *up = vs.uvw + 3 * irow;
     const double W = up[2];
-    const double tu = dadd(up[0], dmul(W, f.cu)), tv = dadd(up[1], dmul(W, f.cv));
+    const double tu = dadd(up[0], dmul(W, cu)), tv = dadd(up[1], dmul(W, cv));
     const unsigned char *fl = vs.flags + irow * vs.nchan * (int64_t)vs.ncorr;
     for (int ch = ch0; ch < ch1; ++ch) {
       if (fl[(int64_t)ch * vs.ncorr]) continue;
@@ -400,6 +440,26 @@ __device__ __forceinline__ BlockMeans grid_block_means(const ddfg_vis &vs, const
       m.last_ch = ch;
       ++m.nvis;
     }
+  }
+  return m;
+}
+
+__device__ __forceinline__ BlockMeans grid_block_means(const ddfg_vis &vs, const ddfg_facet &f, int64_t b) {
+  const int64_t start = vs.block_start[b];
+  return grid_block_sums(vs, f.cu, f.cv, vs.bda_map + start + 2, vs.bda_map[2 + b] - 2, vs.bda_map[start],
+                         vs.bda_map[start + 1]);
+}
+
+// The same divided by the number of visibilities.
+__device__ __forceinline__ BlockMeans block_means_i(const ddfg_vis &vs, double cu, double cv, const int32_t *rows,
+                                                    int nrows, int ch0, int ch1) {
+  BlockMeans m = grid_block_sums(vs, cu, cv, rows, nrows, ch0, ch1);
+  if (m.nvis > 1) {  // x / 1.0 == x exactly
+    const double dn = (double)m.nvis;
+    m.u = m.u / dn;
+    m.v = m.v / dn;
+    m.w = m.w / dn;
+    m.nu = m.nu / dn;
   }
   return m;
 }

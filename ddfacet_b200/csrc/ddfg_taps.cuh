@@ -1,328 +1,670 @@
-// Warp-cooperative tap loops shared by the gridding, degridding and adjoint kernels.
+// Warp-cooperative tap loops: laying a warp's records onto a facet grid (scatter) and gathering a
+// warp's footprints from a model grid.
+//
+// A record is a block's footprint (S x S cells at an origin), its tap table and its values.  The
+// lanes take its taps t = lane + 32 k; SLOTS taps a lane and pass, so footprints of more than 32
+// SLOTS taps are walked in several passes and SLOTS sets registers, not the largest support.
+// Records travel through the warp's shared memory (broadcast loads) instead of through four to six
+// shuffles each, compacted so that the loops run over valid records only, four in flight: their
+// loads are issued first, then their products in order.  Records of different supports (W planes
+// of one stripe) are walked support by support.
 #pragma once
+#include <type_traits>
+
 #include "ddfg_common.cuh"
 #include "ddfg_gridblock.cuh"
 
 namespace ddfg {
 
-// Warp-cooperative tap scatter of the warp's 32 records onto facet f (gridder.h:353-362): each
-// record's footprint, CF offset and support travel in three shuffles; each lane keeps the cell
-// offsets of its taps for as long as the support and grid width stay the same.  Up to four
-// records of equal support are issued together so their CF loads are in flight at once.
-// CONJ lays down conj(CF) (the adjoint of the degridder's gather).  Must be called by all 32
-// lanes.
-template <int NPOL, int SLOTS, bool CONJ = false>
-__device__ __forceinline__ void scatter_records(const GridRecord<NPOL> &rec, const ddfg_facet &f, int npol_used,
-                                                LaneTaps<SLOTS> &lt, int lane) {
-  float2 *grid = (float2 *)f.grid;
-  const float2 *cfd = (const float2 *)f.cf_data;
-  const int plane_sz = f.nx * f.ny;
-  TapJob job;
-  if (rec.valid) job = tap_job(rec.g, rec.gridchan, f);
-  unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
-  if (!mask) return;
-  // Fast path: every valid record of the stripe has the same support, which fits the slots (the
-  // usual case: a stripe is one row's channels, all on one W plane).  The lane's tap pointers
-  // are formed once, and each record costs three shuffles, its CF loads and the reductions.
-  const int first = __ffs(mask) - 1;
-  const int s_inv0 = __shfl_sync(0xffffffffu, rec.valid ? job.s_inv : 0, first);
-  const int S0 = s_inv0 & 255;
-  if (S0 * S0 <= 32 * SLOTS && __all_sync(0xffffffffu, !rec.valid || (job.s_inv & 255) == S0)) {
-    lt.set(s_inv0, f.nx, lane);
-    const float2 *cf_lane = cfd + lane;
-    float2 *g_lane[SLOTS];
-    bool on[SLOTS];
+// Taps a lane and pass for the largest support of a launch: supports up to 8 fit two; wider ones take
+// four, or two where the Stokes planes multiply the registers.
+inline int tap_slots(int max_support, int npol) { return max_support <= 8 || npol > 2 ? 2 : 4; }
+
+// Row t / S of tap t < S^2 (S <= 63); any value in range for taps past the footprint.
+__device__ __forceinline__ int tap_row(int t, int S) {
+  return __float2int_rz(__fdividef((float)t + 0.5f, (float)S));
+}
+
+// ----------------------------------------------------------------------------------------
+// Scatter, one Stokes plane: runs in registers, stripes in a shared-memory tile
+// ----------------------------------------------------------------------------------------
+// Consecutive blocks of a map are neighbouring channels or times of one baseline: their footprints
+// coincide in runs and otherwise overlap.  A run is summed in registers; a finished run is added to
+// the warp's tile of shared memory that covers the records' bounding box (plain loads and stores:
+// the lanes of one run own different cells, a __syncwarp orders runs); the tile reaches the grid
+// once, one addition a touched cell.  A B200 takes 120-130 G 32-byte sectors a second of FP64
+// reductions wherever they fall, which bounded the gridder when every run went to the grid (16
+// sectors a record on 256 channels, 31 on 64).
+//
+// The tile holds FP64 sums for a facet with an FP64 accumulator, FP32 sums otherwise, so a run reaches
+// the same sum as it would in the grid.  (FP32 tiles under FP64 grids would be 3 % faster on 256
+// channels and raise the error against 64 bits from 4.9e-8 to 6.4e-8.)  It is kept all zero between
+// uses: what adds it to the grid clears it.  Its pitch is a multiple of 16 (FP64: 8) cells plus the
+// support where that fits: the rows of a footprint then fall on distinct banks.
+template <int CELLS>
+struct alignas(16) TileSmem {
+  double2 tile[CELLS];
+  int4 rec[32];  // byte offset of the footprint's origin in the tile, tap table offset, value
+};
+
+// Shared-memory accesses by 32-bit address.
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ float2 lds_f2(unsigned a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ double2 lds_d2(unsigned a) {
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ double lds_d(unsigned a) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ int4 lds_i4(unsigned a) {
+  int4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts_f2(unsigned a, float2 v) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts_d2(unsigned a, double2 v) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts_d(unsigned a, double v) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// *p += v unless v is zero.
+__device__ __forceinline__ void red_add_f64(double *p, double v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.neu.f64 p, %1, 0d0000000000000000;\n\t@p red.global.add.f64 [%0], %1;\n\t}" ::"l"(
+                   p),
+               "d"(v)
+               : "memory");
+}
+
+// v onto complex128 cell `cell` of acc (none if negative) for every lane of the warp: lanes 2i and
+// 2i+1 swap halves so that each reduction carries whole cells.  A cell's two doubles in one
+// instruction are one sector operation instead of two, and the sectors are what FP64 reductions
+// cost: 7 x 7 footprints, 249 G cells/s against 126 G cells/s with one instruction for the real and
+// one for the imaginary parts.
+__device__ __forceinline__ void red_add_cells_f64(double *acc, int cell, float2 v, int lane) {
+  const bool odd = lane & 1;
+  const float got = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
+  const int other = __shfl_xor_sync(0xffffffffu, cell, 1);
+  const int ca = odd ? other : cell, cb = odd ? cell : other;
+  double *d = acc + (lane & 1);
+  if (ca >= 0) red_add_f64(d + 2 * (size_t)ca, odd ? got : v.x);
+  if (cb >= 0) red_add_f64(d + 2 * (size_t)cb, odd ? v.y : got);
+}
+
+// Adds the products of n records (a multiple of four) of support S to the tile, taps first ..
+// first + 32 SLOTS - 1.  Bit j of runs: record j starts a run.  F64: an FP64 tile; RUN64: the runs'
+// sums in FP64 too (of products rounded to FP32).
+template <int SLOTS, bool CONJ, bool F64, bool RUN64>
+__device__ __forceinline__ void tile_pass(unsigned tile, unsigned recs, int n, unsigned runs, int S, int first,
+                                          int pitch, const float2 *cfd, int lane) {
+  bool on[SLOTS];
+  unsigned cell[SLOTS];
+  using Sum = typename std::conditional<RUN64, double2, float2>::type;
+  Sum acc[SLOTS];
+  float2 c[4][SLOTS];
+#pragma unroll
+  for (int k = 0; k < SLOTS; ++k) {
+    const int t = first + lane + 32 * k, sy = tap_row(t, S);
+    on[k] = t < S * S;
+    cell[k] = tile + (F64 ? 16 : 8) * (sy * pitch + t - sy * S);
+    acc[k].x = acc[k].y = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) c[r][k] = czero();
+  }
+  cfd += first + lane;
+  unsigned cur = 0;
+  auto flush = [&]() {  // the run's sums to the tile
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < SLOTS; ++k) {
-      on[k] = lt.off[k] >= 0;
-      g_lane[k] = grid + (on[k] ? lt.off[k] : 0);
+      const unsigned a = cell[k] + cur;
+      if (on[k]) {
+        if (F64) {
+          const double2 t = lds_d2(a);
+          sts_d2(a, make_double2(t.x + (double)acc[k].x, t.y + (double)acc[k].y));
+        } else {
+          const float2 t = lds_f2(a);
+          sts_f2(a, make_float2(t.x + (float)acc[k].x, t.y + (float)acc[k].y));
+        }
+      }
+      acc[k].x = acc[k].y = 0;
     }
-    while (mask) {
-      int src[4];
-      int nr = 0;
+  };
+  for (int i = 0; i < n; i += 4) {
+    int4 q[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        src[r] = mask ? __ffs(mask) - 1 : src[0];
-        if (mask) {
-          mask &= mask - 1;
-          ++nr;
-        }
-      }
-      int base[4], cfo[4];
-      float2 sv[4][NPOL];
+    for (int r = 0; r < 4; ++r) {
+      q[r] = lds_i4(recs + 16 * (i + r));
+      const float2 *p = cfd + q[r].y;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        base[r] = __shfl_sync(0xffffffffu, job.base, src[r]);
-        cfo[r] = __shfl_sync(0xffffffffu, job.cfoff, src[r]);
+      for (int k = 0; k < SLOTS; ++k)
+        if (on[k]) c[r][k] = __ldg(p + 32 * k);
+    }
 #pragma unroll
-        for (int p = 0; p < NPOL; ++p) {
-          sv[r][p].x = __shfl_sync(0xffffffffu, rec.stokes[p].x, src[r]);
-          sv[r][p].y = __shfl_sync(0xffffffffu, rec.stokes[p].y, src[r]);
-        }
-      }
-      float2 c[4][SLOTS];
+    for (int r = 0; r < 4; ++r) {
+      if (runs >> (i + r) & 1) flush();  // the same for all lanes
+      cur = q[r].x;
+      const float2 v = make_float2(__int_as_float(q[r].z), __int_as_float(q[r].w));
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int k = 0; k < SLOTS; ++k) c[r][k] = on[k] ? __ldg(cf_lane + cfo[r] + 32 * k) : czero();
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        if (r < nr) {
-#pragma unroll
-          for (int k = 0; k < SLOTS; ++k) {
-            if (on[k]) {
-              float2 *cell = g_lane[k] + base[r];
-#pragma unroll
-              for (int p = 0; p < NPOL; ++p)
-                if (NPOL == 1 || p < npol_used) red_add(cell + (size_t)p * plane_sz, cmul(sv[r][p], CONJ ? cconj(c[r][k]) : c[r][k]));
-            }
-          }
+      for (int k = 0; k < SLOTS; ++k) {
+        if constexpr (RUN64) {
+          const float2 t = cmul(CONJ ? cconj(c[r][k]) : c[r][k], v);
+          acc[k].x += (double)t.x;
+          acc[k].y += (double)t.y;
+        } else {
+          acc[k] = CONJ ? cfma_conj(c[r][k], v, acc[k]) : cfma(c[r][k], v, acc[k]);
         }
       }
     }
-    return;
   }
+  flush();
+  __syncwarp();
+}
+
+// Adds the tile's bw x bh cells to the grid at cell `origin` and clears them, row by row.
+__device__ __forceinline__ void tile_to_grid(unsigned tile, int bw, int bh, int pitch, const ddfg_facet &f,
+                                             size_t origin, int lane) {
+  if (f.grid_acc) {
+    // a lane a double: a cell's two halves in one instruction are one sector operation
+    for (int j = lane; j < 2 * bw; j += 32) {
+      unsigned t = tile + 8 * j;
+      double *d = (double *)f.grid_acc + 2 * origin + j;
+#pragma unroll 4
+      for (int r = 0; r < bh; ++r) {
+        const double v = lds_d(t);
+        sts_d(t, 0.);
+        red_add_f64(d, v);
+        t += 16 * pitch;
+        d += 2 * (ptrdiff_t)f.nx;
+      }
+    }
+  } else {
+    for (int j = lane; j < bw; j += 32) {
+      unsigned t = tile + 8 * j;
+      float2 *d = (float2 *)f.grid + origin + j;
+#pragma unroll 4
+      for (int r = 0; r < bh; ++r) {
+        const float2 v = lds_f2(t);
+        sts_f2(t, czero());
+        if (v.x != 0.f || v.y != 0.f) red_add(d, v);
+        t += 8 * pitch;
+        d += f.nx;
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// Adds the warp's 32 records to facet f (gridder.h:353-362): into the FP64 accumulator when the
+// facet has one, else into the float32 grid.  CONJ lays down conj(CF) (the adjoint of the
+// degridder's gather).  sm: the warp's own, its tile zero.  Must be called by all 32 lanes.
+// BLOCKS: averaged blocks, whose runs are long (0.1 cells a block) -- an FP64 accumulator gets FP64
+// runs; single visibilities' runs of about three are summed in FP32 as they always were.
+template <int SLOTS, bool CONJ, bool BLOCKS, int CELLS>
+__device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddfg_facet &f, TileSmem<CELLS> &sm,
+                                             int lane) {
+  const unsigned tile = smem_addr(sm.tile), recs = smem_addr(sm.rec);
+  unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
+  const int bx = rec.g.locx - rec.g.sup, by = rec.g.locy - rec.g.sup;
   while (mask) {
-    int src[4];
-    int nr = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      src[r] = mask ? __ffs(mask) - 1 : -1;
-      if (mask) {
-        mask &= mask - 1;
-        ++nr;
+    // the records of one support and band, as many (in lane order) as the tile covers
+    const int lead = __ffs(mask) - 1;
+    const int S = __shfl_sync(0xffffffffu, rec.g.S, lead), band = __shfl_sync(0xffffffffu, rec.gridchan, lead);
+    unsigned seg = __ballot_sync(0xffffffffu, rec.valid && rec.g.S == S && rec.gridchan == band) & mask;
+    int x0, y0, bw, bh;
+    for (;;) {
+      const bool in = (seg >> lane) & 1;
+      x0 = __reduce_min_sync(0xffffffffu, in ? bx : 0x7fffffff);
+      y0 = __reduce_min_sync(0xffffffffu, in ? by : 0x7fffffff);
+      bw = __reduce_max_sync(0xffffffffu, in ? bx : -1) - x0 + S;
+      bh = __reduce_max_sync(0xffffffffu, in ? by : -1) - y0 + S;
+      if (bw * bh <= CELLS || (seg & (seg - 1)) == 0) break;
+      const int mid = (lead + 31 - __clz(seg)) >> 1;  // the lower half of its lanes
+      seg &= (2u << mid) - 1u;
+    }
+    mask &= ~seg;
+    const size_t origin = ((size_t)(band * f.npol) * f.ny + y0) * f.nx + x0;
+    const float2 *const cfd = (const float2 *)f.cf_data;
+    if (bw * bh > CELLS) {  // one record with a support too wide for the tile: tap by tap
+      const int cfo = __shfl_sync(0xffffffffu, rec.g.cfoff, lead);
+      const float2 s = make_float2(__shfl_sync(0xffffffffu, rec.stokes[0].x, lead),
+                                   __shfl_sync(0xffffffffu, rec.stokes[0].y, lead));
+      for (int t = lane; t < ((S * S + 31) & ~31); t += 32) {
+        const bool on = t < S * S;
+        const float2 c = on ? __ldg(cfd + cfo + t) : czero();
+        const float2 v = cmul(s, CONJ ? cconj(c) : c);
+        const int cell = t / S * f.nx + t % S;
+        if (f.grid_acc) red_add_cells_f64((double *)f.grid_acc + 2 * origin, on ? cell : -1, v, lane);
+        else if (on) red_add((float2 *)f.grid + origin + cell, v);
+      }
+      continue;
+    }
+    const bool f64 = f.grid_acc != nullptr;
+    int pitch = bw + ((S - bw) & (f64 ? 7 : 15));
+    if (pitch * bh > CELLS) pitch = bw;
+    const int n = __popc(seg), n4 = (n + 3) & ~3;
+    if ((seg >> lane) & 1) {
+      const int at = __popc(seg & ((1u << lane) - 1u));
+      const float2 s = rec.stokes[0];
+      const int to = (f64 ? 16 : 8) * ((by - y0) * pitch + bx - x0);
+      sm.rec[at] = make_int4(to, rec.g.cfoff, __float_as_int(s.x), __float_as_int(s.y));
+      if (at == n - 1)  // copies of the last record with a zero value fill the last group of four
+        for (int j = n; j < n4; ++j) sm.rec[j] = make_int4(to, rec.g.cfoff, 0, 0);
+    }
+    __syncwarp();
+    const unsigned runs =
+        __ballot_sync(0xffffffffu, lane > 0 && lane < n && sm.rec[lane].x != sm.rec[lane > 0 ? lane - 1 : 0].x);
+    const int step = SLOTS == 2 || S <= 8 ? 64 : 32 * SLOTS;
+    for (int first = 0; first < S * S; first += step) {
+      if (SLOTS == 2 || S <= 8) {
+        if (f64) tile_pass<2, CONJ, true, BLOCKS>(tile, recs, n4, runs, S, first, pitch, cfd, lane);
+        else tile_pass<2, CONJ, false, false>(tile, recs, n4, runs, S, first, pitch, cfd, lane);
+      } else {
+        if (f64) tile_pass<SLOTS, CONJ, true, BLOCKS>(tile, recs, n4, runs, S, first, pitch, cfd, lane);
+        else tile_pass<SLOTS, CONJ, false, false>(tile, recs, n4, runs, S, first, pitch, cfd, lane);
       }
     }
-    TapJob j[4];
-    float2 sv[4][NPOL];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int sr = src[r] >= 0 ? src[r] : src[0];
-      j[r] = shfl_job(job, sr);
-#pragma unroll
-      for (int p = 0; p < NPOL; ++p) {
-        sv[r][p].x = __shfl_sync(0xffffffffu, rec.stokes[p].x, sr);
-        sv[r][p].y = __shfl_sync(0xffffffffu, rec.stokes[p].y, sr);
-      }
-    }
-    const int S = j[0].s_inv & 255;
-    bool same = S * S <= 32 * SLOTS;
-#pragma unroll
-    for (int r = 1; r < 4; ++r) same = same && (r >= nr || (j[r].s_inv & 255) == S);
-    if (same) {
-      lt.set(j[0].s_inv, f.nx, lane);
-      float2 c[4][SLOTS];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int k = 0; k < SLOTS; ++k)
-          c[r][k] = (r < nr && lt.off[k] >= 0) ? __ldg(cfd + j[r].cfoff + lane + 32 * k) : czero();
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        if (r >= nr) break;
-#pragma unroll
-        for (int k = 0; k < SLOTS; ++k) {
-          if (lt.off[k] >= 0) {
-            float2 *cell = grid + (j[r].base + lt.off[k]);
-#pragma unroll
-            for (int p = 0; p < NPOL; ++p)
-              if (p < npol_used) red_add(cell + (size_t)p * plane_sz, cmul(sv[r][p], CONJ ? cconj(c[r][k]) : c[r][k]));
-          }
-        }
-      }
-    } else {
-      for (int r = 0; r < nr; ++r) {
-        const int Sr = j[r].s_inv & 255;
-        const unsigned inv = (unsigned)j[r].s_inv >> 8;
-        for (int t = lane; t < Sr * Sr; t += 32) {
-          const int sy = (int)(((unsigned)t * inv) >> 16);
-          const float2 cv = __ldg(cfd + j[r].cfoff + t);
-          float2 *cell = grid + (j[r].base + sy * f.nx + (t - sy * Sr));
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p)
-            if (p < npol_used) red_add(cell + (size_t)p * plane_sz, cmul(sv[r][p], CONJ ? cconj(cv) : cv));
-        }
-      }
-    }
+    tile_to_grid(tile, bw, bh, pitch, f, origin, lane);
   }
 }
 
-// Lane partial sums of the warp's 32 blocks, staged in shared memory and reduced by column:
-// lane j adds the 32 partials of block j (one pass instead of a butterfly per block).
-constexpr int kPartialBytesPerWarp = 32 * 32 * 8;
+// ----------------------------------------------------------------------------------------
+// Scatter, several Stokes planes: the footprint in registers as a torus
+// ----------------------------------------------------------------------------------------
+// A tile would need a plane's space four times; the planes share tap loads and addresses, so here
+// the registers do the merging.  A lane owns the torus positions t (t < S^2): of any S x S window
+// exactly one cell (x, y) has (y mod S) S + (x mod S) = t, so the lane's cell for the next record is
+// the same one as long as the window still covers it.  The lane keeps adding into registers and
+// reaches memory only when the window leaves its cell: a move by one column costs S additions a
+// plane, not S^2.  (A facet with an FP64 accumulator still takes every run.)
 
-// Cooperative gather of every valid record's taps on facet f (degridder.h:202-212): four
-// records of equal support at once, lanes on consecutive taps of a CF row; the sum of record r
-// ends in lane r's mine[].  For one Stokes plane the lane partials are reduced through the
-// warp's shared-memory tile wpart (one column per record); otherwise by butterflies.
-// Must be called by all 32 lanes.
-template <int NPOL, int SLOTS>
-__device__ __forceinline__ void gather_records(bool valid, const TapJob &job, const ddfg_facet &f,
-                                               LaneTaps<SLOTS> &lt, float2 *wpart, int lane, float2 *mine) {
-#pragma unroll
-  for (int p = 0; p < NPOL; ++p) mine[p] = czero();
-  const int plane_sz = f.nx * f.ny;
-  const float2 *grid = (const float2 *)f.grid;
-  const float2 *cfd = (const float2 *)f.cf_data;
-  const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-  unsigned mask = vmask;
-  // Fast path: every valid record has the same support, which fits the slots: the lane's tap
-  // pointers are formed once; each record costs two shuffles and its CF and model loads.
-  const int first = mask ? __ffs(mask) - 1 : 0;
-  const int s_inv0 = __shfl_sync(0xffffffffu, valid ? job.s_inv : 0, first);
-  const int S0 = s_inv0 & 255;
-  if (mask && S0 * S0 <= 32 * SLOTS && __all_sync(0xffffffffu, !valid || (job.s_inv & 255) == S0)) {
-    lt.set(s_inv0, f.nx, lane);
-    const float2 *cf_lane = cfd + lane;
-    const float2 *g_lane[SLOTS];
-    bool on[SLOTS];
+// x mod S for 0 <= x < 2^26, magic = torus_magic(S).
+__device__ __forceinline__ unsigned torus_magic(int S) { return 0xffffffffu / (unsigned)S + 1u; }
+__device__ __forceinline__ int torus_mod(int x, int S, unsigned magic) {
+  return S > 1 ? x - (int)__umulhi((unsigned)x, magic) * S : 0;
+}
+
+// A lane's torus positions of one pass and their place in the current window.
+template <int SLOTS>
+struct TorusLane {
+  int cx[SLOTS], cy[SLOTS];
+  bool on[SLOTS];
+  int off[SLOTS];   // tap index (row-major in the window) of the position
+  int cell[SLOTS];  // its cell index in the grid, -1 for positions past S^2
+  __device__ __forceinline__ void set(int S, int first) {
 #pragma unroll
     for (int k = 0; k < SLOTS; ++k) {
-      on[k] = lt.off[k] >= 0;
-      g_lane[k] = grid + (on[k] ? lt.off[k] : 0);
-    }
-    while (mask) {
-      int src[4];
-      int nr = 0;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        src[r] = mask ? __ffs(mask) - 1 : src[0];
-        if (mask) {
-          mask &= mask - 1;
-          ++nr;
-        }
-      }
-      int base[4], cfo[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        base[r] = __shfl_sync(0xffffffffu, job.base, src[r]);
-        cfo[r] = __shfl_sync(0xffffffffu, job.cfoff, src[r]);
-      }
-      float2 c[4][SLOTS], gv[4][SLOTS][NPOL];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int k = 0; k < SLOTS; ++k) {
-          c[r][k] = on[k] ? __ldg(cf_lane + cfo[r] + 32 * k) : czero();
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p)
-            gv[r][k][p] = on[k] ? __ldg(g_lane[k] + base[r] + (size_t)p * plane_sz) : czero();
-        }
-      float2 acc[4][NPOL];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int p = 0; p < NPOL; ++p) {
-          acc[r][p] = czero();
-#pragma unroll
-          for (int k = 0; k < SLOTS; ++k) acc[r][p] = cadd(acc[r][p], cmul(gv[r][k][p], c[r][k]));
-        }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        if (r >= nr) break;
-        if (NPOL == 1) {
-          wpart[src[r] * 32 + lane] = acc[r][0];
-        } else {
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-              acc[r][p].x += __shfl_xor_sync(0xffffffffu, acc[r][p].x, o);
-              acc[r][p].y += __shfl_xor_sync(0xffffffffu, acc[r][p].y, o);
-            }
-          }
-          if (lane == src[r]) {
-#pragma unroll
-            for (int p = 0; p < NPOL; ++p) mine[p] = acc[r][p];
-          }
-        }
-      }
+      const int t = first + 32 * k;
+      on[k] = t < S * S;
+      const int tt = on[k] ? t : 0;  // idle positions read tap 0 and never reach the grid
+      cy[k] = tap_row(tt, S);
+      cx[k] = tt - cy[k] * S;
+      cell[k] = -1;
+      off[k] = 0;
     }
   }
-  while (mask) {
-    // Up to four records of equal support at once: their CF and grid loads overlap.
-    int src[4];
-    int nr = 0;
+  // Moves the window to the origin with cell index base and (bx mod S, by mod S) = (m & 255, m >> 8).
+  __device__ __forceinline__ void move(int base, int m, int S, int nx) {
+    const int mx = m & 255, my = m >> 8;
+#pragma unroll
+    for (int k = 0; k < SLOTS; ++k) {
+      const int dx = cx[k] - mx, dy = cy[k] - my;
+      const int tx = (int)min((unsigned)dx, (unsigned)(dx + S)), ty = (int)min((unsigned)dy, (unsigned)(dy + S));
+      off[k] = ty * S + tx;
+      cell[k] = on[k] ? base + ty * nx + tx : -1;
+    }
+  }
+};
+
+template <int NPOL>
+struct alignas(16) TorusSmem {
+  int4 rec[32];  // cell index of the window's origin, tap table offset, the first Stokes value
+  int mod[32];
+  float2 st[NPOL > 1 ? NPOL - 1 : 1][32];
+};
+
+// One pass of the torus over n records (n a multiple of four) of support S.
+template <int NPOL, int SLOTS, bool CONJ>
+__device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int S, int first,
+                                             const ddfg_facet &f, int npol_used, int lane) {
+  float2 *const grid = (float2 *)f.grid;
+  double *const acc64 = (double *)f.grid_acc;
+  const float2 *const cfd = (const float2 *)f.cf_data;
+  const int nx = f.nx;
+  const size_t plane = (size_t)f.nx * f.ny;
+  TorusLane<SLOTS> tl;
+  tl.set(S, first + lane);
+  int cell[SLOTS];  // the cells the sums below belong to
+  float2 a[NPOL][SLOTS];
+#pragma unroll
+  for (int k = 0; k < SLOTS; ++k) {
+    cell[k] = -1;
+#pragma unroll
+    for (int p = 0; p < NPOL; ++p) a[p][k] = czero();
+  }
+  auto flush = [&](int k, int to) {  // slot k's sums to cell `to` (-1: this lane has none to flush)
+#pragma unroll
+    for (int p = 0; p < NPOL; ++p) {
+      if (p >= npol_used) break;
+      if (acc64) red_add_cells_f64(acc64 + 2 * p * plane, to, a[p][k], lane);
+      else if (to >= 0) red_add(grid + p * plane + to, a[p][k]);
+    }
+  };
+  int cur = -1, ahead = -1;  // origin of the sums, origin of the records being loaded
+  for (int i = 0; i < n; i += 4) {
+    int4 q[4];
+    float2 c[4][SLOTS];
+    int to[4][SLOTS];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      src[r] = mask ? __ffs(mask) - 1 : -1;
-      if (mask) {
-        mask &= mask - 1;
-        ++nr;
+      q[r] = sm.rec[i + r];
+      if (q[r].x != ahead) {  // the same for all lanes
+        ahead = q[r].x;
+        tl.move(ahead, sm.mod[i + r], S, nx);
+      }
+#pragma unroll
+      for (int k = 0; k < SLOTS; ++k) {
+        to[r][k] = tl.cell[k];
+        c[r][k] = __ldg(cfd + (q[r].y + tl.off[k]));
       }
     }
-    TapJob j[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) j[r] = shfl_job(job, src[r] >= 0 ? src[r] : src[0]);
-    const int S = j[0].s_inv & 255;
-    bool same = S * S <= 32 * SLOTS;
-#pragma unroll
-    for (int r = 1; r < 4; ++r) same = same && (r >= nr || (j[r].s_inv & 255) == S);
-    float2 acc[4][NPOL];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int p = 0; p < NPOL; ++p) acc[r][p] = czero();
-    if (same) {
-      lt.set(j[0].s_inv, f.nx, lane);
-      float2 c[4][SLOTS], gv[4][SLOTS][NPOL];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r) {
+      if (q[r].x != cur) {
+        cur = q[r].x;
 #pragma unroll
         for (int k = 0; k < SLOTS; ++k) {
-          const bool on = r < nr && lt.off[k] >= 0;
-          c[r][k] = on ? __ldg(cfd + j[r].cfoff + lane + 32 * k) : czero();
+          // FP64 sums take every run by itself, as FP64 additions did before runs merged
+          const bool leave = acc64 || to[r][k] != cell[k];
+          flush(k, leave ? cell[k] : -1);
+          if (leave) {
+            cell[k] = to[r][k];
 #pragma unroll
-          for (int p = 0; p < NPOL; ++p)
-            gv[r][k][p] = on ? __ldg(grid + (j[r].base + lt.off[k]) + (size_t)p * plane_sz) : czero();
+            for (int p = 0; p < NPOL; ++p) a[p][k] = czero();
+          }
         }
+      }
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int p = 0; p < NPOL; ++p) {
+        const float2 v = p == 0 ? make_float2(__int_as_float(q[r].z), __int_as_float(q[r].w)) : sm.st[p > 0 ? p - 1 : 0][i + r];
 #pragma unroll
         for (int k = 0; k < SLOTS; ++k)
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) acc[r][p] = cadd(acc[r][p], cmul(gv[r][k][p], c[r][k]));
-    } else {
-      for (int r = 0; r < nr; ++r) {
-        const int Sr = j[r].s_inv & 255;
-        const unsigned inv = (unsigned)j[r].s_inv >> 8;
-        for (int t = lane; t < Sr * Sr; t += 32) {
-          const int sy = (int)(((unsigned)t * inv) >> 16);
-          const float2 cv = __ldg(cfd + j[r].cfoff + t);
-          const float2 *cell = grid + (j[r].base + sy * f.nx + (t - sy * Sr));
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) acc[r][p] = cadd(acc[r][p], cmul(__ldg(cell + (size_t)p * plane_sz), cv));
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (r >= nr) break;
-      if (NPOL == 1) {
-        wpart[src[r] * 32 + lane] = acc[r][0];
-      } else {
-#pragma unroll
-        for (int p = 0; p < NPOL; ++p) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            acc[r][p].x += __shfl_xor_sync(0xffffffffu, acc[r][p].x, o);
-            acc[r][p].y += __shfl_xor_sync(0xffffffffu, acc[r][p].y, o);
-          }
-        }
-        if (lane == src[r]) {
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) mine[p] = acc[r][p];
-        }
+          a[p][k] = CONJ ? cfma_conj(c[r][k], v, a[p][k]) : cfma(c[r][k], v, a[p][k]);
       }
     }
   }
-  if (NPOL == 1) {
+#pragma unroll
+  for (int k = 0; k < SLOTS; ++k) flush(k, cell[k]);
+}
+
+// Adds the warp's 32 records to facet f (gridder.h:353-362): into the FP64 accumulator when the
+// facet has one, else into the float32 grid.  CONJ lays down conj(CF) (the adjoint of the
+// degridder's gather).  sm: the warp's own.  Must be called by all 32 lanes.
+template <int NPOL, int SLOTS, bool CONJ = false>
+__device__ __forceinline__ void scatter_torus(const GridRecord<NPOL> &rec, const ddfg_facet &f, int npol_used,
+                                              TorusSmem<NPOL> &sm, int lane) {
+  unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
+  while (mask) {
+    const int S = __shfl_sync(0xffffffffu, rec.g.S, __ffs(mask) - 1);
+    const bool mine = rec.valid && rec.g.S == S;
+    const unsigned sub = __ballot_sync(0xffffffffu, mine);
+    mask &= ~sub;
+    const int n = __popc(sub), n4 = (n + 3) & ~3;
+    int base = 0, mod = 0, cfo = 0;
+    if (mine) {
+      const int bx = rec.g.locx - rec.g.sup, by = rec.g.locy - rec.g.sup;
+      const unsigned magic = torus_magic(S);
+      base = ((rec.gridchan * f.npol) * f.ny + by) * f.nx + bx;
+      mod = torus_mod(bx, S, magic) | torus_mod(by, S, magic) << 8;
+      cfo = rec.g.cfoff;
+      const int at = __popc(sub & ((1u << lane) - 1u));
+      sm.rec[at] = make_int4(base, cfo, __float_as_int(rec.stokes[0].x), __float_as_int(rec.stokes[0].y));
+      sm.mod[at] = mod;
+#pragma unroll
+      for (int p = 1; p < NPOL; ++p) sm.st[p > 0 ? p - 1 : 0][at] = rec.stokes[p];
+    }
+    // up to three copies of the last record with zero values fill the last group of four
+    const int last = 31 - __clz(sub);
+    base = __shfl_sync(0xffffffffu, base, last);
+    cfo = __shfl_sync(0xffffffffu, cfo, last);
+    mod = __shfl_sync(0xffffffffu, mod, last);
+    if (lane < n4 - n) {
+      sm.rec[n + lane] = make_int4(base, cfo, 0, 0);
+      sm.mod[n + lane] = mod;
+#pragma unroll
+      for (int p = 1; p < NPOL; ++p) sm.st[p > 0 ? p - 1 : 0][n + lane] = czero();
+    }
     __syncwarp();
-    if (valid) {
-      float2 t = czero();
-#pragma unroll 8
-      for (int i = 0; i < 32; ++i) t = cadd(t, wpart[lane * 32 + ((i + lane) & 31)]);
-      mine[0] = t;
+    if (SLOTS > 2 && S <= 8) {
+      torus_pass<NPOL, 2, CONJ>(sm, n4, S, 0, f, npol_used, lane);
+    } else {
+      for (int first = 0; first < S * S; first += 32 * SLOTS)
+        torus_pass<NPOL, SLOTS, CONJ>(sm, n4, S, first, f, npol_used, lane);
+    }
+    __syncwarp();
+  }
+}
+
+template <int NPOL, int SLOTS>
+struct ScatterSmem {
+  TorusSmem<NPOL> torus;
+  __device__ __forceinline__ void clear(int) {}
+};
+// Tiles of 22 x 22 cells for supports up to 8 (a 7 x 7 footprint's travel of 15 cells), 25 x 25
+// for wider ones: two CTAs of eight warps an SM.
+template <int SLOTS>
+struct ScatterSmem<1, SLOTS> {
+  static constexpr int kCells = SLOTS == 2 ? 512 : 640;
+  TileSmem<kCells> tile;
+  __device__ __forceinline__ void clear(int lane) {
+    for (int i = lane; i < kCells; i += 32) tile.tile[i] = make_double2(0., 0.);
+    __syncwarp();
+  }
+};
+
+// The warp's records onto facet f.  sm: the warp's own, cleared once (clear) before the first call.
+template <int NPOL, int SLOTS, bool CONJ = false, bool BLOCKS = false>
+__device__ __forceinline__ void scatter(const GridRecord<NPOL> &rec, const ddfg_facet &f, int npol_used,
+                                        ScatterSmem<NPOL, SLOTS> &sm, int lane) {
+  if constexpr (NPOL == 1) scatter_tile<SLOTS, CONJ, BLOCKS>(rec, f, sm.tile, lane);
+  else scatter_torus<NPOL, SLOTS, CONJ>(rec, f, npol_used, sm.torus, lane);
+}
+
+// ----------------------------------------------------------------------------------------
+// Gather
+// ----------------------------------------------------------------------------------------
+// A run of records with one footprint origin loads its model cells once and keeps them in
+// registers; every record costs its tap loads, its products and one partial sum a lane.
+
+template <int NPOL>
+struct alignas(16) GatherSmem {
+  float2 part[8][32];    // lane partial sums of eight (record, plane) rows
+  float2 out[32][NPOL];  // sums
+  int2 rec[32];          // cell index of the footprint's origin, tap table offset
+};
+
+// The 8 rows of sm.part summed over lanes: four lanes a row, each over eight partials (read so that
+// a quarter warp's 16-byte loads fall on distinct banks), then two shuffles.  Lanes 4 j get row j.
+__device__ __forceinline__ float2 sum_rows(const float2 (*part)[32], int lane) {
+  const int row = lane >> 2, quarter = lane & 3;
+  const float4 *p = (const float4 *)&part[row][quarter * 8];
+  float2 t = czero();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 v = p[(i + (quarter >> 1) + 2 * row) & 3];
+    t = cadd(t, make_float2(v.x + v.z, v.y + v.w));
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+    t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+  }
+  return t;
+}
+
+// The lane partials of records i .. i + GROUP - 1 to their rows of sm.part; with the last rows of a
+// reduction, their sums to sm.out.
+template <int NPOL, int GROUP>
+__device__ __forceinline__ void gather_store(GatherSmem<NPOL> &sm, const float2 (*t)[NPOL], int i, int n, int lane) {
+  constexpr int ROWS = 8 / NPOL;  // records of one reduction: 8, 4, 2, 2
+#pragma unroll
+  for (int r = 0; r < GROUP; ++r)
+#pragma unroll
+    for (int p = 0; p < NPOL; ++p) sm.part[((i + r) % ROWS) * NPOL + p][lane] = t[r][p];
+  if ((i + GROUP) % ROWS == 0 || i + GROUP >= n) {
+    __syncwarp();
+    const float2 v = sum_rows(sm.part, lane);
+    const int row = lane >> 2, rec = i / ROWS * ROWS + row / NPOL;
+    if ((lane & 3) == 0 && row < ROWS * NPOL && rec < n) sm.out[rec][row % NPOL] = v;
+    __syncwarp();
+  }
+}
+
+// Sums n records (a multiple of four) of support S <= 8: a run's model cells stay in registers.
+template <int NPOL>
+__device__ __forceinline__ void gather_narrow(GatherSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, int lane) {
+  constexpr int GROUP = NPOL == 1 ? 4 : NPOL == 2 ? 4 : 2;  // records in flight
+  const size_t plane = (size_t)f.nx * f.ny;
+  bool on[2];
+  const float2 *cell[2];
+  float2 held[NPOL][2], c[GROUP][2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int t = lane + 32 * k, sy = tap_row(t, S);
+    on[k] = t < S * S;
+    cell[k] = (const float2 *)f.grid + (sy * f.nx + t - sy * S);
+#pragma unroll
+    for (int p = 0; p < NPOL; ++p) held[p][k] = czero();
+#pragma unroll
+    for (int r = 0; r < GROUP; ++r) c[r][k] = czero();
+  }
+  const float2 *const cfd = (const float2 *)f.cf_data + lane;
+  int cur = -1;
+  for (int i = 0; i < n; i += GROUP) {
+    float2 g[GROUP][NPOL][2], t[GROUP][NPOL];
+    bool moved[GROUP];
+#pragma unroll
+    for (int r = 0; r < GROUP; ++r) {
+      const int2 q = sm.rec[i + r];
+      moved[r] = q.x != cur;  // the same for all lanes
+      if (moved[r]) {
+        cur = q.x;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p) g[r][p][k] = on[k] ? __ldg(cell[k] + cur + p * plane) : czero();
+      }
+      const float2 *p = cfd + q.y;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (on[k]) c[r][k] = __ldg(p + 32 * k);
+    }
+#pragma unroll
+    for (int r = 0; r < GROUP; ++r) {
+      if (moved[r]) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p) held[p][k] = g[r][p][k];
+      }
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) t[r][p] = cfma(c[r][1], held[p][1], cmul(c[r][0], held[p][0]));
+    }
+    gather_store<NPOL, GROUP>(sm, t, i, n, lane);
+  }
+}
+
+// The same for any support: four records at a time over all their taps, 32 SLOTS a round, so that a
+// record still costs one partial sum a lane.  Records of a round on one origin share its cells.
+template <int NPOL, int SLOTS>
+__device__ __forceinline__ void gather_wide(GatherSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, int lane) {
+  constexpr int GROUP = NPOL <= 2 ? 4 : 2;
+  const size_t plane = (size_t)f.nx * f.ny;
+  const float2 *const cfd = (const float2 *)f.cf_data + lane;
+  const float2 *const grid = (const float2 *)f.grid;
+  const int row0 = tap_row(lane, S), col0 = lane - row0 * S, drow = tap_row(32, S), dcol = 32 - drow * S;
+  for (int i = 0; i < n; i += GROUP) {
+    int2 q[GROUP];
+    float2 t[GROUP][NPOL];
+#pragma unroll
+    for (int r = 0; r < GROUP; ++r) {
+      q[r] = sm.rec[i + r];
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) t[r][p] = czero();
+    }
+    int row = row0, col = col0;
+    for (int first = 0; first < S * S; first += 32 * SLOTS) {
+      float2 c[GROUP][SLOTS], g[NPOL][SLOTS];
+      int at[SLOTS];
+#pragma unroll
+      for (int k = 0; k < SLOTS; ++k) {
+        const bool on = first + 32 * k + lane < S * S;
+        at[k] = on ? row * f.nx + col : -1;
+        col += dcol;
+        row += drow;
+        if (col >= S) {
+          col -= S;
+          ++row;
+        }
+#pragma unroll
+        for (int r = 0; r < GROUP; ++r) c[r][k] = on ? __ldg(cfd + q[r].y + first + 32 * k) : czero();
+      }
+#pragma unroll
+      for (int r = 0; r < GROUP; ++r) {
+        if (r == 0 || q[r].x != q[r > 0 ? r - 1 : 0].x) {  // the same for all lanes
+#pragma unroll
+          for (int k = 0; k < SLOTS; ++k)
+#pragma unroll
+            for (int p = 0; p < NPOL; ++p) g[p][k] = at[k] >= 0 ? __ldg(grid + q[r].x + at[k] + p * plane) : czero();
+        }
+#pragma unroll
+        for (int p = 0; p < NPOL; ++p)
+#pragma unroll
+          for (int k = 0; k < SLOTS; ++k) t[r][p] = cfma(c[r][k], g[p][k], t[r][p]);
+      }
+    }
+    gather_store<NPOL, GROUP>(sm, t, i, n, lane);
+  }
+}
+
+// The sums over every valid record's taps on facet f (degridder.h:202-212); the sum of lane r's
+// record ends in its mine[].  sm: the warp's own.  Must be called by all 32 lanes.
+template <int NPOL, int SLOTS>
+__device__ __forceinline__ void gather(bool valid, const BlockGeom &g, int gridchan, const ddfg_facet &f,
+                                       GatherSmem<NPOL> &sm, int lane, float2 *mine) {
+#pragma unroll
+  for (int p = 0; p < NPOL; ++p) mine[p] = czero();
+  unsigned mask = __ballot_sync(0xffffffffu, valid);
+  while (mask) {
+    const int S = __shfl_sync(0xffffffffu, g.S, __ffs(mask) - 1);
+    const bool own = valid && g.S == S;
+    const unsigned sub = __ballot_sync(0xffffffffu, own);
+    mask &= ~sub;
+    const int n = __popc(sub), n4 = (n + 3) & ~3;
+    const int at = __popc(sub & ((1u << lane) - 1u));
+    if (own) {
+      const int2 q = make_int2(((gridchan * f.npol) * f.ny + g.locy - g.sup) * f.nx + g.locx - g.sup, g.cfoff);
+      sm.rec[at] = q;
+      if (at == n - 1)  // copies of the last record fill the last group of four
+        for (int j = n; j < n4; ++j) sm.rec[j] = q;
+    }
+    __syncwarp();
+    if (S <= 8) gather_narrow<NPOL>(sm, n4, S, f, lane);
+    else gather_wide<NPOL, SLOTS>(sm, n4, S, f, lane);
+    if (own) {
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) mine[p] = sm.out[at][p];
     }
     __syncwarp();
   }

@@ -364,12 +364,11 @@ def make_pol(corr_ids, stokes_ids) -> _abi.Pol:
 
 @dataclass
 class Batch:
-    """Scheduling of the batched (persistent, queue-driven) calls and their workspace
-    (ddfg_batch): facets per pack, stripes per queue item, resident CTAs per SM (0 = library
-    default); ``static`` replaces the queue by a fixed item order (for measurements), ``tiles``
-    has the gridder's warps sum each stripe in a shared-memory tile before adding it to the grid,
-    and ``spread`` interleaves the items over one contiguous region of the block order per CTA
-    (concurrent CTAs work on distant parts of a uv-ordered map)."""
+    """Scheduling of the batched (persistent) calls and their workspace (ddfg_batch): facets per
+    pack, stripes of a CTA's chunk, resident CTAs per SM (0 = library default); ``static`` replaces
+    the queue by a fixed order (for measurements), ``spread`` gives each CTA neighbouring chunks
+    (concurrent CTAs work on distant parts of a uv-ordered map); ``tiles`` is accepted and has no
+    effect (the gridder always sums a stripe in a shared-memory tile)."""
     workspace: torch.Tensor
     facets_per_pack: int = 0
     stripes_per_item: int = 0

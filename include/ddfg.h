@@ -142,24 +142,23 @@ typedef struct ddfg_pol {
 } ddfg_pol;
 
 /* Scheduling of ddfg_grid_batched / ddfg_degrid_batched: one persistent launch per call (per
- * DDFG_TABLE_FACETS facets) whose CTAs take work items from a queue in device memory.  An item
- * is a run of stripes (32 consecutive blocks) of one facet pack; the warps of a CTA apply every
- * facet of the pack to a stripe in turn (its inputs are read once per pack).  Items are ordered
- * pack by pack, the large-block items of a pack first (the longest work starts first).  Zero
- * fields take the library's defaults (or the autotuner's choice, ddfacet_b200.autotune). */
+ * DDFG_TABLE_FACETS facets) that walks the facets pack by pack.  A warp applies every facet of a pack
+ * to a stripe (32 consecutive blocks) in turn (its inputs are read once per pack).  The warps of a
+ * CTA share chunks of consecutive stripes; the last fifth of the stripes, and the large blocks
+ * before everything else, come from a queue in device memory.  Zero fields take the library's
+ * defaults (or the autotuner's choice, ddfacet_b200.autotune). */
 typedef struct ddfg_batch {
   void *workspace;             /* >= ddfg_batch_workspace_size() bytes of device scratch, 8-byte aligned */
   size_t workspace_bytes;
   int32_t facets_per_pack;     /* facets applied to a stripe before the next stripe (0: default) */
-  int32_t stripes_per_item;    /* stripes of one queue item (0: default)                   */
+  int32_t stripes_per_item;    /* stripes of a CTA's chunk (0: default)                    */
   int32_t ctas_per_sm;         /* resident CTAs per SM of the persistent launch (0: occupancy) */
-  int32_t flags;               /* bit 0: static item order instead of the queue (for
-                                  measurements); bit 1: the gridder's warps sum each stripe into a
-                                  shared-memory tile and add the touched cells to the grid once
-                                  (one Stokes plane; pays when a stripe's footprints overlap);
-                                  bit 2: spread the items over as many contiguous regions of the
-                                  block order as the launch has CTAs, taken in turn (CTAs work far
-                                  apart: for maps in uv-cell order, on distant grid cells) */
+  int32_t flags;               /* bit 0: round robin instead of the queue (for measurements);
+                                  bit 1: accepted, without effect (the gridder always sums a stripe
+                                  in a shared-memory tile where it has one Stokes plane);
+                                  bit 2: a CTA's chunks are neighbours in the block order instead of
+                                  interleaved with the other CTAs' (for maps in uv-cell order: CTAs
+                                  work on distant grid cells) */
 } ddfg_batch;
 
 /* Library and device checks. */
@@ -304,7 +303,7 @@ int ddfg_bda_plan_noalloc(const int32_t *bda_map, int64_t bda_len, int64_t nbloc
 /* Bytes of device scratch ddfg_grid_batched / ddfg_degrid_batched need (the queue counters). */
 size_t ddfg_batch_workspace_size(void);
 
-/* ddfg_grid as one persistent, queue-driven launch per DDFG_TABLE_FACETS facets (see
+/* ddfg_grid as one persistent, scheduled launch per DDFG_TABLE_FACETS facets (see
  * ddfg_batch): same inputs, outputs and checks.  The work queue balances uneven facets and
  * blocks (averaged BDA blocks of very different sizes) across the GPU; every call first resets
  * its counters (one cudaMemsetAsync), so the call can be captured in a CUDA graph.  Replaces the
