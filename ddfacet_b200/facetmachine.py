@@ -230,31 +230,16 @@ class FacetMachine:
         image = torch.zeros((self.nband, self.npol, m, m), dtype=torch.float32, device=self.device)
         for f in self.facets:
             n = f.grid.grid.shape[-1]
-            _abi.check(lib.ddfg_grid_to_image(self._plan(n), C.c_void_p(f.grid.grid.data_ptr()),
-                                              C.c_double(float(self.overs) ** 2),
-                                              C.c_void_p(self._work_for(n).data_ptr()), st))
-            w = self._norm_weights(f)
             xc, yc = f.geom.pix_central
-            _abi.check(lib.ddfg_stitch_facet(C.c_void_p(f.grid.grid.data_ptr()), self.nband, self.npol, n,
-                                             C.c_void_p(f.sphe.data_ptr()), C.c_void_p(f.invsphe.data_ptr()),
-                                             C.c_void_p(f.sw_grid.data_ptr()), C.c_void_p(w.data_ptr()),
-                                             C.c_void_p(image.data_ptr()), m, xc, yc, st))
-        if bool((self.facet_norm_host != 0).any()):
+            _abi.check(lib.ddfg_facet_to_image(self._plan(n), f.grid.grid.data_ptr(), float(self.overs) ** 2, self.nband,
+                                               self.npol, f.sphe.data_ptr(), f.invsphe.data_ptr(),
+                                               f.sw_grid.data_ptr(), f.grid.sumwt.data_ptr(),
+                                               f.grid.sumjones.data_ptr(), image.data_ptr(), m, xc, yc,
+                                               self._work_for(n).data_ptr(), st))
+        if any(row.any() for row in self.facet_norm_host):  # ends at the first row with a facet
             _abi.check(lib.ddfg_image_normalise(C.c_void_p(image.data_ptr()), self.nband * self.npol, m,
                                                 C.c_void_p(self.facet_norm.data_ptr()), st))
         return image
-
-    def _norm_weights(self, f):
-        """SumWeights[band][pol] * sqrt(SumJonesNorm[band]) (ClassFacetMachine.py:1066-1076, 1385-1391)."""
-        sw = f.grid.sumwt
-        sj = f.grid.sumjones
-        if float(sj.abs().sum().item()) == 0.0:
-            norm = torch.ones(self.nband, dtype=torch.float64, device=self.device)
-        else:
-            den = torch.where(sj[1] == 0, torch.ones_like(sj[1]), sj[1])
-            norm = sj[0] / den
-            norm = torch.where(norm == 0, torch.ones_like(norm), norm)
-        return (sw * torch.sqrt(norm)[:, None]).contiguous()
 
     def image_to_facets(self, model_image: torch.Tensor, stream=None, out: Optional[List[torch.Tensor]] = None):
         """Every facet's model grid from the model image float32 [nband, npol, M, M]

@@ -372,6 +372,16 @@ int ddfg_stitch_facet(const void *dirty, int32_t nband, int32_t npol, int32_t n,
                       const float *invsphe, const float *sw_grid, const double *weights, float *image, int32_t m,
                       int32_t xc, int32_t yc, void *stream);
 
+/* ddfg_grid_to_image and ddfg_stitch_facet of one facet, the stitching fused with the transform's last
+ * shift: grid [nband][npol][N][N] becomes the dirty facet image and is added into image.  The
+ * planes' weights are formed on the device: sumwt[band][pol] * sqrt(sumjones[0][band] /
+ * sumjones[1][band]) (a zero divisor or quotient counts as 1; sumjones NULL or all zero: sumwt alone),
+ * as FacetsToIm forms them (ClassFacetMachine.py:1066-1076, 1385-1391).  work: a [nband][npol][N][N]
+ * complex64 scratch buffer. */
+int ddfg_facet_to_image(ddfg_fft_plan *plan, void *grid, double scale, int32_t nband, int32_t npol, const float *sphe,
+                        const float *invsphe, const float *sw_grid, const double *sumwt, const double *sumjones,
+                        float *image, int32_t m, int32_t xc, int32_t yc, void *work, void *stream);
+
 /* image[plane] /= facet_norm (ClassFacetMachine.py:1411-1414); facet_norm is [M][M]. */
 int ddfg_image_normalise(float *image, int32_t planes, int32_t m, const float *facet_norm, void *stream);
 
