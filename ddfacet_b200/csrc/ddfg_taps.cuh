@@ -209,47 +209,68 @@ __device__ __forceinline__ void tile_to_grid(unsigned tile, int bw, int bh, int 
 // Adds the warp's 32 records to facet f (gridder.h:353-362): into the FP64 accumulator when the
 // facet has one, else into the float32 grid.  CONJ lays down conj(CF) (the adjoint of the
 // degridder's gather).  sm: the warp's own, its tile zero.  Must be called by all 32 lanes.
+// Segments of up to this many records skip the tile (10,800 visibilities of 8 channels on one facet,
+// channels up to 12 cells apart, with the window below: 32 us to 22 us).
+constexpr int kFewRecords = 2;
+
 // BLOCKS: averaged blocks, whose runs are long (0.1 cells a block) -- an FP64 accumulator gets FP64
 // runs; single visibilities' runs of about three are summed in FP32 as they always were.
 template <int SLOTS, bool CONJ, bool BLOCKS, int CELLS>
 __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddfg_facet &f, TileSmem<CELLS> &sm,
                                              int lane) {
   const unsigned tile = smem_addr(sm.tile), recs = smem_addr(sm.rec);
+  constexpr int W = CELLS >= 625 ? 25 : 22;  // W x W cells fit
+  static_assert(W * W <= CELLS, "tile");
   unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
   const int bx = rec.g.locx - rec.g.sup, by = rec.g.locy - rec.g.sup;
   while (mask) {
-    // the records of one support and band, as many (in lane order) as the tile covers
+    // the records of one support and band that the tile covers together
     const int lead = __ffs(mask) - 1;
     const int S = __shfl_sync(0xffffffffu, rec.g.S, lead), band = __shfl_sync(0xffffffffu, rec.gridchan, lead);
-    unsigned seg = __ballot_sync(0xffffffffu, rec.valid && rec.g.S == S && rec.gridchan == band) & mask;
-    int x0, y0, bw, bh;
-    for (;;) {
-      const bool in = (seg >> lane) & 1;
+    const bool like = (mask >> lane & 1) && rec.g.S == S && rec.gridchan == band;
+    unsigned seg = __ballot_sync(0xffffffffu, like);
+    int x0 = __reduce_min_sync(0xffffffffu, like ? bx : 0x7fffffff);
+    int y0 = __reduce_min_sync(0xffffffffu, like ? by : 0x7fffffff);
+    int bw = __reduce_max_sync(0xffffffffu, like ? bx : -1) - x0 + S;
+    int bh = __reduce_max_sync(0xffffffffu, like ? by : -1) - y0 + S;
+    if (bw * bh > CELLS) {
+      // not all of them: those in a W x W window that starts a cell behind the first record and
+      // opens towards the last one (a baseline's records move one way)
+      const int last = 31 - __clz(seg), slack = W - S > 1 ? 1 : 0;
+      const int lx = __shfl_sync(0xffffffffu, bx, lead), ly = __shfl_sync(0xffffffffu, by, lead);
+      const int xa = __shfl_sync(0xffffffffu, bx, last) >= lx ? lx - slack : lx + slack - (W - S);
+      const int ya = __shfl_sync(0xffffffffu, by, last) >= ly ? ly - slack : ly + slack - (W - S);
+      const bool in = like && (W < S ? lane == lead : (unsigned)(bx - xa) <= (unsigned)(W - S) &&
+                                                          (unsigned)(by - ya) <= (unsigned)(W - S));
+      seg = __ballot_sync(0xffffffffu, in);
       x0 = __reduce_min_sync(0xffffffffu, in ? bx : 0x7fffffff);
       y0 = __reduce_min_sync(0xffffffffu, in ? by : 0x7fffffff);
       bw = __reduce_max_sync(0xffffffffu, in ? bx : -1) - x0 + S;
       bh = __reduce_max_sync(0xffffffffu, in ? by : -1) - y0 + S;
-      if (bw * bh <= CELLS || (seg & (seg - 1)) == 0) break;
-      const int mid = (lead + 31 - __clz(seg)) >> 1;  // the lower half of its lanes
-      seg &= (2u << mid) - 1u;
     }
     mask &= ~seg;
-    const size_t origin = ((size_t)(band * f.npol) * f.ny + y0) * f.nx + x0;
     const float2 *const cfd = (const float2 *)f.cf_data;
-    if (bw * bh > CELLS) {  // one record with a support too wide for the tile: tap by tap
-      const int cfo = __shfl_sync(0xffffffffu, rec.g.cfoff, lead);
-      const float2 s = make_float2(__shfl_sync(0xffffffffu, rec.stokes[0].x, lead),
-                                   __shfl_sync(0xffffffffu, rec.stokes[0].y, lead));
-      for (int t = lane; t < ((S * S + 31) & ~31); t += 32) {
-        const bool on = t < S * S;
-        const float2 c = on ? __ldg(cfd + cfo + t) : czero();
-        const float2 v = cmul(s, CONJ ? cconj(c) : c);
-        const int cell = t / S * f.nx + t % S;
-        if (f.grid_acc) red_add_cells_f64((double *)f.grid_acc + 2 * origin, on ? cell : -1, v, lane);
-        else if (on) red_add((float2 *)f.grid + origin + cell, v);
+    if (bw * bh > CELLS || (!BLOCKS && __popc(seg) <= kFewRecords)) {
+      // a support wider than the tile, or too few records to pay for it: tap by tap
+      for (; seg; seg &= seg - 1) {
+        const int src = __ffs(seg) - 1;
+        const float2 *const taps = cfd + __shfl_sync(0xffffffffu, rec.g.cfoff, src);
+        const float2 s = make_float2(__shfl_sync(0xffffffffu, rec.stokes[0].x, src),
+                                     __shfl_sync(0xffffffffu, rec.stokes[0].y, src));
+        const size_t at = ((size_t)(band * f.npol) * f.ny + __shfl_sync(0xffffffffu, by, src)) * f.nx +
+                          __shfl_sync(0xffffffffu, bx, src);
+        for (int t = lane; t < ((S * S + 31) & ~31); t += 32) {
+          const bool on = t < S * S;
+          const float2 c = on ? __ldg(taps + t) : czero();
+          const float2 v = cmul(s, CONJ ? cconj(c) : c);
+          const int sy = tap_row(t, S), cell = sy * f.nx + t - sy * S;
+          if (f.grid_acc) red_add_cells_f64((double *)f.grid_acc + 2 * at, on ? cell : -1, v, lane);
+          else if (on) red_add((float2 *)f.grid + at + cell, v);
+        }
       }
       continue;
     }
+    const size_t origin = ((size_t)(band * f.npol) * f.ny + y0) * f.nx + x0;
     const bool f64 = f.grid_acc != nullptr;
     int pitch = bw + ((S - bw) & (f64 ? 7 : 15));
     if (pitch * bh > CELLS) pitch = bw;
