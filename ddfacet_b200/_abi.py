@@ -146,6 +146,8 @@ def lib_path() -> str:
 def lib():
     """Load (building if needed) libddfg.so; raise if it cannot be loaded."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             path = _build.LIB
