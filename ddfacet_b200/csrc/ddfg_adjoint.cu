@@ -716,7 +716,7 @@ int launch_i(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet *facets,
   const int rc = ddfg_kernel_prepare(kern, 256, smem, &per_sm);
   if (rc) return rc;
   const int ctas = ddfg_num_ctas(per_sm);
-  sched_split(sc, nullptr, ctas, 8);
+  sched_split(sc, nullptr, ctas, 8, false);
   if (grad) jones_grad_single_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, sc, grad);
   else adjoint_single_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, sc);
   const cudaError_t e = cudaGetLastError();

@@ -346,7 +346,7 @@ int launch_degrid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTab
   if (rc) return rc;
   if (batch && batch->ctas_per_sm > 0) per_sm = min(per_sm, (int)batch->ctas_per_sm);
   const int ctas = ddfg_num_ctas(per_sm);
-  sched_split(sc, batch, ctas, 8);
+  sched_split(sc, batch, ctas, 8, !single);
   if (stokes_i && single) degrid_single_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, dp, sc);
   else if (stokes_i) degrid_block_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, dp, sc);
   else if (single) degrid_single_q<NP, SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, dp, sc);

@@ -463,7 +463,7 @@ int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable
   if (rc) return rc;
   if (batch && batch->ctas_per_sm > 0) per_sm = min(per_sm, (int)batch->ctas_per_sm);
   const int ctas = ddfg_num_ctas(per_sm);
-  sched_split(sc, batch, ctas, threads / 32);
+  sched_split(sc, batch, ctas, threads / 32, !single);
   if (stokes_i && single) grid_single_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (stokes_i) grid_block_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (single) grid_single_q<NP, SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);

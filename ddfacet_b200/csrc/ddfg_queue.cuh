@@ -43,10 +43,12 @@ struct Sched {
 };
 
 // Host: the chunks and items of a launch of ctas CTAs of `warps` warps.  batch->stripes_per_item
-// sets the chunk (0: 64 stripes, or an eighth of a CTA's where that is less).
-inline void sched_split(Sched &sc, const ddfg_batch *batch, int ctas, int warps) {
+// sets the chunk (0: 64 stripes of single visibilities, 16 of averaged blocks, whose stripes differ so
+// much that longer chunks leave CTAs behind -- averaged gridding 42.9 ms with 64, 35.2 with 16; 256
+// channels 26.3 with 64, 27.1 with 16 -- or an eighth of a CTA's stripes where that is less).
+inline void sched_split(Sched &sc, const ddfg_batch *batch, int ctas, int warps, bool averaged) {
   const long long per_cta = sc.nstripes / ctas;
-  long long chunk = batch && batch->stripes_per_item > 0 ? batch->stripes_per_item : 64;
+  long long chunk = batch && batch->stripes_per_item > 0 ? batch->stripes_per_item : averaged ? 16 : 64;
   if (chunk > per_cta / 8) chunk = per_cta / 8;
   if (chunk < warps) chunk = warps;
   sc.chunk = (int)chunk;
