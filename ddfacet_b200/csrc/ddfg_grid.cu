@@ -496,14 +496,15 @@ int ddfg_launch_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet 
   const int acc_stride = nwarps_cta * max_band + (chan_sums ? 2 * vs->nchan : 0);
   const size_t per_facet_smem = grid_facet_smem(nwarps_cta, acc_stride, nvispol == 1 && grid_is_i(vs, js, gp), single);
   // Shared memory per CTA: two 256-thread CTAs (single-visibility maps) or three 128-thread CTAs
-  // (averaged blocks) per SM, each with the warps' grid tiles (one Stokes plane) and the shared
-  // accumulators of a pack.
-  const size_t budget = single ? 110 * 1024 : 74 * 1024;
+  // (averaged blocks) per SM, each with its warps' tiles and the shared sums of a pack -- or one CTA per
+  // SM where the sums of one facet (hundreds of bands, thousands of channels) need more.
   const size_t scatter_smem = nvispol == 1   ? (slots == 2 ? grid_smem<1, 2>(nwarps_cta) : grid_smem<1, 4>(nwarps_cta))
                               : nvispol == 2 ? grid_smem<2, 2>(nwarps_cta)
                               : nvispol == 3 ? grid_smem<3, 2>(nwarps_cta)
                                              : grid_smem<4, 2>(nwarps_cta);
-  const int max_fit = (int)((budget - scatter_smem) / per_facet_smem);
+  size_t budget = single ? 110 * 1024 : 74 * 1024;
+  if (budget < scatter_smem + per_facet_smem) budget = 225 * 1024;
+  const int max_fit = budget < scatter_smem + per_facet_smem ? 0 : (int)((budget - scatter_smem) / per_facet_smem);
   if (max_fit < 1) return ddfg_set_error(DDFG_ESIZE, "grid: too many bands/channels for the shared accumulators");
   int want = (batch && batch->facets_per_pack > 0) ? batch->facets_per_pack : 16;
   want = max(1, min(want, max_fit));

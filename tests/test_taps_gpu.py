@@ -103,3 +103,17 @@ def test_stokes_i_kernels_against_general(form, ncorr, nchan, nch):
             grads.append(torch.autograd.grad(p, [grid, kms], grad_outputs=vs.vis))
         for a, b in zip(*grads):
             assert _rms(a, b) < 1e-6
+
+
+@pytest.mark.parametrize("kw", [dict(nchan=160, nband=150), dict(nchan=3000, nband=2, bda_mode=1, dphi=0.5)],
+                         ids=["bands", "channels"])
+def test_sums_that_fill_shared_memory(kw):
+    """One facet's weight sums (150 bands, eight warps) or per-channel Jones sums (3000 channels) beside
+    the wide tiles: more shared memory than two or three CTAs an SM leave each other."""
+    c = cases.make_case(seed=47, nant=4, ntimes=4, ncorr=4, npix=125, cell_arcsec=5.0, nw=2, sup=11, **kw)
+    cases.add_jones(c, nt=2, nd=2, mode=1)
+    want = cases.run_fp64_grid(c)
+    got = cases.run_gpu_grid(c, batched=True, fp64_acc=True)
+    assert cases.rel_rms(got["grid"], want["grid"]) < 1e-6
+    np.testing.assert_allclose(got["sumwt"], want["sumwt"], rtol=1e-12)
+    np.testing.assert_allclose(got["sumjones_chan"], want["sumjones_chan"], rtol=1e-5)
