@@ -21,8 +21,8 @@
 // What bounds them (256 channels, 16 facets a pack, 310 M facet-visibilities): the L1 data path (73 %
 // of its wavefronts: four for a record's taps, five when its model cells change, four for its lane
 // partials) and issue (63 %, 30 instructions a record); 28.3 ms before records went through shared
-// memory, runs kept their model cells and Stokes I had kernels of its own (ddfg_single.cuh), 23.7 ms
-// now.  Averaged blocks (9 uneven facets): 23.9 ms to 15.9 ms, on the latency of the block walks.
+// memory, runs kept their model cells and Stokes I had kernels of its own (ddfg_single.cuh), 23.9 ms
+// now.  Averaged blocks (9 uneven facets): 24.3 ms to 15.2 ms, on the latency of the block walks.
 #include <cuda_runtime.h>
 
 #include "ddfg_common.cuh"
@@ -331,7 +331,7 @@ namespace {
 
 template <int NP, int SL>
 int launch_degrid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable &tab, const DegridParams &dp,
-                        Sched sc, const ddfg_batch *batch, cudaStream_t stream) {
+                        Sched sc, const ddfg_batch *batch, bool &zeroed, int counters, cudaStream_t stream) {
   const bool single = vs->single_vis_blocks != 0;
   const bool stokes_i = NP == 1 && dp.policy == D_DIAG_FROM_I && !vs->uvw_dt && jones_as_stored(js) &&
                         (single || js->mode != 2);
@@ -347,6 +347,7 @@ int launch_degrid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTab
   if (batch && batch->ctas_per_sm > 0) per_sm = min(per_sm, (int)batch->ctas_per_sm);
   const int ctas = ddfg_num_ctas(per_sm);
   sched_split(sc, batch, ctas, 8, !single);
+  if ((rc = sched_counters(sc, true, ctas * 8, zeroed, counters, stream))) return rc;
   if (stokes_i && single) degrid_single_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, dp, sc);
   else if (stokes_i) degrid_block_i<SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, dp, sc);
   else if (single) degrid_single_q<NP, SL><<<ctas, 256, smem, stream>>>(*vs, *js, tab, dp, sc);
@@ -371,13 +372,9 @@ int ddfg_launch_degrid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_face
   const int per_launch = (batch && batch->facets_per_pack > 0) ? min((int)batch->facets_per_pack, DDFG_TABLE_FACETS)
                                                                : DDFG_TABLE_FACETS;
   const int ngroups = (nfacets + per_launch - 1) / per_launch;  // <= DDFG_MAX_FACETS
-  unsigned int *counters = nullptr;
-  if (batch && !(batch->flags & 1)) {
-    // counters after the gridder's (a grid and a degrid call may share one workspace)
-    counters = (unsigned int *)batch->workspace + kGridCounters;
-    const cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned int) * ngroups, stream);
-    if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "degrid: %s", cudaGetErrorString(e));
-  }
+  // counters after the gridder's (a grid and a degrid call may share one workspace)
+  unsigned int *counters = batch && !(batch->flags & 1) ? (unsigned int *)batch->workspace + kGridCounters : nullptr;
+  bool zeroed = false;
   const long long nstripes = (vs->nblocks + 31) / 32;
   const int nlarge = vs->single_vis_blocks ? 0 : (int)(vs->nlarge < (1LL << 30) ? vs->nlarge : (1LL << 30));
   FacetTable tab;
@@ -396,7 +393,7 @@ int ddfg_launch_degrid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_face
     sc.large_items = nlarge;
     sc.counter = counters ? counters + g : nullptr;
     int rc;
-#define LD(NP, SL) rc = launch_degrid_table<NP, SL>(vs, js, tab, dp, sc, batch, stream)
+#define LD(NP, SL) rc = launch_degrid_table<NP, SL>(vs, js, tab, dp, sc, batch, zeroed, ngroups - g, stream)
     if (slots == 2) {
       switch (nvispol) {
         case 1: LD(1, 2); break;

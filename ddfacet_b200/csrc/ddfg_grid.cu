@@ -26,9 +26,9 @@
 //
 // What bounds them (256 channels, 25 facets of 1485^2, 310 M facet-visibilities, FP64 sums): 38.5 ms
 // with a reduction per tap and run, on the FP64 reduction rate of L2 (16 sectors a record, 125 G
-// sectors/s); now 26.5 ms at 48 instructions and 3.8 sectors a record, on instruction issue (51 %)
+// sectors/s); now 26.4 ms at 48 instructions and 3.8 sectors a record, on instruction issue (51 %)
 // and the shared-memory / L1 data path (57 %) together -- 24 warps an SM instead of 16 change
-// nothing.  64 channels, 735^2: 16.6 ms to 8.0 ms.
+// nothing.  64 channels, 735^2: 16.7 ms to 8.1 ms.
 #include <cuda_runtime.h>
 
 #include "ddfg_common.cuh"
@@ -451,7 +451,7 @@ size_t grid_facet_smem(int warps, int acc_stride, bool stokes_i, bool single) {
 
 template <int NP, int SL>
 int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable &tab, const GridParams &gp,
-                      Sched sc, const ddfg_batch *batch, cudaStream_t stream) {
+                      Sched sc, const ddfg_batch *batch, bool &zeroed, int counters, cudaStream_t stream) {
   const bool single = vs->single_vis_blocks != 0, stokes_i = NP == 1 && grid_is_i(vs, js, gp);
   const int threads = single ? 256 : 128;
   const size_t smem = grid_smem<NP, SL>(threads / 32) +
@@ -464,6 +464,7 @@ int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable
   if (batch && batch->ctas_per_sm > 0) per_sm = min(per_sm, (int)batch->ctas_per_sm);
   const int ctas = ddfg_num_ctas(per_sm);
   sched_split(sc, batch, ctas, threads / 32, !single);
+  if ((rc = sched_counters(sc, false, ctas * (threads / 32), zeroed, counters, stream))) return rc;
   if (stokes_i && single) grid_single_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (stokes_i) grid_block_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (single) grid_single_q<NP, SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
@@ -508,13 +509,9 @@ int ddfg_launch_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet 
   if (max_fit < 1) return ddfg_set_error(DDFG_ESIZE, "grid: too many bands/channels for the shared accumulators");
   int want = (batch && batch->facets_per_pack > 0) ? batch->facets_per_pack : 16;
   want = max(1, min(want, max_fit));
-  unsigned int *counters = nullptr;  // one a pack
+  unsigned int *counters = batch && !(batch->flags & 1) ? (unsigned int *)batch->workspace : nullptr;  // one a pack
+  bool zeroed = false;
   const int ngroups = (nfacets + DDFG_TABLE_FACETS - 1) / DDFG_TABLE_FACETS;
-  if (batch && !(batch->flags & 1)) {
-    counters = (unsigned int *)batch->workspace;
-    const cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned int) * nfacets, stream);
-    if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "grid: %s", cudaGetErrorString(e));
-  }
   const long long nstripes = (vs->nblocks + 31) / 32;
   const int nlarge = vs->single_vis_blocks ? 0 : (int)(vs->nlarge < (1LL << 30) ? vs->nlarge : (1LL << 30));
   FacetTable tab_tl;  // host staging of the parameter table (copied into the launch)
@@ -533,7 +530,7 @@ int ddfg_launch_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet 
     sc.large_items = nlarge;
     sc.counter = counters ? counters + f0 : nullptr;  // a launch has at most as many packs as facets
     int rc;
-#define LG(NP, SL) rc = launch_grid_table<NP, SL>(vs, js, tab_tl, gp, sc, batch, stream)
+#define LG(NP, SL) rc = launch_grid_table<NP, SL>(vs, js, tab_tl, gp, sc, batch, zeroed, nfacets - f0, stream)
     if (slots == 2) {
       switch (nvispol) {
         case 1: LG(1, 2); break;

@@ -402,7 +402,7 @@ __device__ __forceinline__ void warp_add_single_sums(const ddfg_vis &vs, const d
 // memory.  Straight to global memory, 32 neighbouring channels are 16 sectors a stripe and facet and
 // a shared copy (4 KB a facet at 256 channels) would cost the tile its room; with few channels every
 // warp of the GPU adds to the same few sectors (16 channels, one facet, 340,000 visibilities: 230 us
-// against 60 us with shared copies).
+// a call without shared copies, most of it waiting there).
 constexpr int kSharedChannels = 128;
 
 // Visibilities of block b (rows x channels, flagged ones included).

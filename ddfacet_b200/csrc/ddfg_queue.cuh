@@ -36,6 +36,7 @@ struct Sched {
   int chunk;                 // stripes of a CTA's chunk
   int chunks;                // chunks a CTA
   int spread;                // 1: a CTA's chunks are neighbours, 0: the CTAs' chunks interleave
+  int near;                  // 1: the CTA's stripes are neighbours and its warps take turns
   long long tail;            // first stripe of the last fifth
   int run;                   // its stripes an item
   long long large_items;     // large blocks
@@ -54,9 +55,29 @@ inline void sched_split(Sched &sc, const ddfg_batch *batch, int ctas, int warps,
   sc.chunk = (int)chunk;
   // a CTA with less than two stripes a warp takes them all one by one
   sc.chunks = per_cta < 2 * warps ? 0 : (int)(per_cta * 4 / (5 * chunk));
+  sc.near = 0;
   sc.spread = batch && (batch->flags & 4) ? 1 : 0;
   sc.tail = (long long)ctas * sc.chunks * sc.chunk;
   sc.run = sc.chunks > 0 && sc.nstripes - sc.tail > 8LL * ctas * warps ? 2 : 1;
+}
+
+// Host: zeroes the counters of a call's launches before the first that uses them (`n` from sc.counter
+// on).  A launch with less than two stripes a warp and no large blocks has nothing to even out: it goes
+// round robin, without the memset and one or two round trips a warp to one address.  Where it gathers
+// and has at least a stripe a warp, a CTA's stripes are neighbours, which share model cells and taps in
+// L1; scattering, neighbours would add to the same cells at once (whole calls with one
+// facet: degridding 223,000 visibilities 50.3 us with the counter, 45.2 round robin, 43.2 with
+// neighbours; gridding 115,000 visibilities 46.2, 46.5 and 50.7).
+inline int sched_counters(Sched &sc, bool gathers, int warps_launched, bool &zeroed, int n, cudaStream_t stream) {
+  if (sc.chunks == 0 && sc.large_items == 0) {
+    sc.counter = nullptr;
+    sc.near = gathers && sc.nstripes >= warps_launched ? 1 : 0;
+  }
+  if (!sc.counter || zeroed) return 0;
+  const cudaError_t e = cudaMemsetAsync(sc.counter, 0, sizeof(unsigned int) * n, stream);
+  if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "queue counters: %s", cudaGetErrorString(e));
+  zeroed = true;
+  return 0;
 }
 
 __device__ __forceinline__ int pack_first(const Sched &sc, int p) {
@@ -110,6 +131,12 @@ struct WarpWork {
         return true;
       }
       phase = 2;
+    }
+    if (sc.near) {
+      const long long hi = (blockIdx.x + 1) * sc.nstripes / gridDim.x;
+      w.s0 = blockIdx.x * sc.nstripes / gridDim.x + (threadIdx.x >> 5) + (blockDim.x >> 5) * seq++;
+      w.s1 = w.s0 + 1;
+      return w.s0 < hi;
     }
     const unsigned int it = held != 0xffffffffu ? held : item(sc, pack, lane);
     held = 0xffffffffu;
