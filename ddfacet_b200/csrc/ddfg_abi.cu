@@ -227,9 +227,13 @@ int ddfg_kernel_prepare(const void *kernel, int threads, size_t smem, int *per_s
     }
   }
   std::lock_guard<std::mutex> lock(g_prep_mutex);
+  // The default limit of 48 KB holds for the kernel's static and dynamic shared memory together.
+  cudaFuncAttributes attr;
+  e = cudaFuncGetAttributes(&attr, kernel);
+  if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "kernel prepare: %s", cudaGetErrorString(e));
   const PrepKey kkey{kernel, dev, 0, 0};
   size_t &limit = g_smem_limit[kkey];
-  if (smem > 48 * 1024 && smem > limit) {
+  if (attr.sharedSizeBytes + smem > 48 * 1024 && smem > limit) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
       return ddfg_set_error(DDFG_ECUDA, "kernel prepare: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));

@@ -20,9 +20,10 @@ int ddfg_one_wave(K kernel, int threads, size_t smem) {
   return ddfg_num_ctas(per_sm);
 }
 
-// Sets the kernel's dynamic shared-memory limit when smem needs more than the default and
-// returns its resident CTAs per SM for (threads, smem) in *per_sm; both are cached per kernel,
-// device and size, so a launch inside a captured step does no repeated host work.
+// Sets the kernel's dynamic shared-memory limit when smem, with the kernel's static shared memory,
+// needs more than the default, and returns its resident CTAs per SM for (threads, smem) in *per_sm;
+// both are cached per kernel, device and size, so a launch inside a captured step does no repeated
+// host work.
 int ddfg_kernel_prepare(const void *kernel, int threads, size_t smem, int *per_sm);
 
 // Queue counters in a ddfg_batch workspace: the gridder's (one per pack, at most one per facet),
