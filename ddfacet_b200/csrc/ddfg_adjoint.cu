@@ -751,13 +751,17 @@ int ddfg_launch_degrid_adjoint(const ddfg_vis *vs, const ddfg_jones *js, const d
     const int f0 = (int)(((long long)ip * nfacets) / npacks);
     FacetPack pack;
     pack.n = (int)(((long long)(ip + 1) * nfacets) / npacks) - f0;
+    // the gradient goes to grid: an FP64 accumulator is the gridder's, and nothing folds it here
+    for (int i = 0; i < pack.n; ++i) {
+      pack.f[i] = facets[f0 + i];
+      pack.f[i].grid_acc = nullptr;
+    }
     if (adjoint_is_i(vs, js, policy)) {
-      const int rc = slots == 2 ? launch_i<2>(vs, js, facets + f0, pack.n, nullptr, stream)
-                                : launch_i<4>(vs, js, facets + f0, pack.n, nullptr, stream);
+      const int rc = slots == 2 ? launch_i<2>(vs, js, pack.f, pack.n, nullptr, stream)
+                                : launch_i<4>(vs, js, pack.f, pack.n, nullptr, stream);
       if (rc) return rc;
       continue;
     }
-    for (int i = 0; i < pack.n; ++i) pack.f[i] = facets[f0 + i];
     int rc;
 #define LAUNCH_A(NP, SL) rc = launch_adjoint<NP, SL>(vs, js, pack, policy, stream)
     if (slots == 2) {

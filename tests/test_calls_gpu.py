@@ -42,3 +42,27 @@ def test_degrid_planes_times_facets(n, stokes, kw):
         out.append(v.vis)
     assert _rms(out[1], out[0]) < 1e-6
     assert _rms(out[2], out[0]) < 1e-6
+
+
+ADJ = {"stokes_i": dict(), "iquv": dict(stokes_ids=(1, 2, 3, 4)), "bda": dict(bda_mode=1, dphi=0.6),
+       "wide": dict(sup=11, stokes_ids=(1, 2))}
+
+
+@pytest.mark.parametrize("form", list(ADJ))
+def test_adjoint_leaves_the_accumulator_alone(form):
+    """ddfg_degrid_adjoint adds to ``grid``; an FP64 accumulator belongs to the gridding calls."""
+    c = cases.make_case(seed=62, nant=7, ntimes=8, nchan=8, ncorr=4, npix=127, cell_arcsec=5.0, nw=2, **ADJ[form])
+    cases.add_jones(c, nt=2, nd=2, mode=1)
+    vs, fg, jd = cases._gpu_objs(c)
+    pol = D.make_pol(c.corr_ids, c.stokes_ids)
+    lib, vss, js = _abi.lib(), vs.struct(), jd.struct()
+    got = []
+    for acc in (None, torch.zeros(fg.grid.shape, dtype=torch.complex128, device="cuda")):
+        g = dataclasses.replace(fg, grid=torch.zeros_like(fg.grid))
+        s = g.struct(degrid=True)
+        s.grid_acc = None if acc is None else acc.data_ptr()
+        _abi.check(lib.ddfg_degrid_adjoint(C.byref(vss), C.byref(js), C.byref(pol), C.byref(s), 1, D._stream_ptr()))
+        got.append(g.grid)
+    assert torch.count_nonzero(torch.view_as_real(acc)) == 0
+    assert torch.count_nonzero(torch.view_as_real(got[0])) > 0
+    assert _rms(got[1], got[0]) < 1e-6  # float32 additions in another order
