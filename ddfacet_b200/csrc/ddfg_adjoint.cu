@@ -671,10 +671,10 @@ __global__ void __launch_bounds__(256, 2) jones_grad_single_i(const ddfg_vis vs,
                            geometry_i(f, dadd(in.U, dmul(in.W, f.cu)), dadd(in.V, dmul(in.W, f.cv)), in.W, in.recip, geo);
         float2 t;
         gather<1, SLOTS>(valid, geo, in.gridchan, sf[fi], ws, lane, &t);
-        t = valid ? cmul(t, phasor_turns(in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * f.n0m1) * kInvC)) : czero();
+        t = cmul(t, phasor_turns(in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * f.n0m1) * kInvC));
         M2 A;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) A.v[p] = cmul(cconj(t), g.v[p]);
+        for (int p = 0; p < 4; ++p) A.v[p] = valid ? cmul(cconj(t), g.v[p]) : czero();  // not 0 x g: g may be NaN
         if (use == 1) {
           if (valid) add_jones_grad_i(js, grad, at.o0 + f.jones_dir, at.o1 + f.jones_dir, A);
         } else {

@@ -66,3 +66,78 @@ def test_adjoint_leaves_the_accumulator_alone(form):
     assert torch.count_nonzero(torch.view_as_real(acc)) == 0
     assert torch.count_nonzero(torch.view_as_real(got[0])) > 0
     assert _rms(got[1], got[0]) < 1e-6  # float32 additions in another order
+
+
+def _geometry(c, vs, fg, degrid=False):
+    """D.block_geometry of a map of single visibilities as [nrow, nchan, 8]."""
+    at = c.bda[2 + vs.nblocks:].reshape(-1, 3)
+    out = np.zeros((c.nrow, c.nchan, 8), np.int32)
+    out[at[:, 2], at[:, 0]] = D.block_geometry(vs, fg, degrid=degrid).cpu().numpy()
+    return out
+
+
+def test_gradients_of_values_that_are_not_finite():
+    """Upstream gradients of NaN and Inf at visibilities that miss the facet (beyond wmax) take no part in
+    the Jones gradient, in the Stokes I kernel as in the general one (reached with smearing switched on and
+    both of its factors off)."""
+    c = cases.make_case(seed=63, nant=7, ntimes=8, nchan=8, ncorr=4, npix=127, cell_arcsec=5.0, nw=3)
+    cases.add_jones(c, nt=2, nd=2, mode=1)
+    vs, fg, jd = cases._gpu_objs(c)
+    fg.cf = dataclasses.replace(fg.cf, wmax=fg.cf.wmax * 0.4)
+    fg = dataclasses.replace(fg, grid=_randn(fg.grid.shape, 3))
+    pol = D.make_pol(c.corr_ids, [1])
+    miss = torch.from_numpy(_geometry(c, vs, fg, degrid=True)[:, :, 0] != 1).cuda()
+    at = torch.nonzero(miss)
+    assert 0.05 * miss.numel() < at.shape[0] < 0.95 * miss.numel()
+    good = vs.vis.clone()
+    good[miss] = 0
+    bad = good.clone()
+    bad[at[::2, 0], at[::2, 1]] = complex(float("nan"), 0.0)
+    bad[at[1::2, 0], at[1::2, 1]] = complex(float("inf"), float("-inf"))
+    lib = _abi.lib()
+    out = []
+    for vis, smear in ((good, False), (bad, False), (bad, True)):
+        v = dataclasses.replace(vs, vis=vis)
+        if smear:
+            v = dataclasses.replace(v, uvw_dt=torch.zeros_like(vs.uvw), dt=1.0, dnu=1.0, do_tsmear=0, do_fsmear=0)
+        kms = torch.zeros_like(jd.kms)
+        vss, js, s = v.struct(), jd.struct(), fg.struct(degrid=True)
+        _abi.check(lib.ddfg_degrid_jones_grad(C.byref(vss), C.byref(js), C.byref(pol), C.byref(s), 1, kms.data_ptr(),
+                                              D._stream_ptr()))
+        out.append(kms)
+    assert torch.isfinite(torch.view_as_real(out[0])).all()
+    for k in out[1:]:
+        assert torch.isfinite(torch.view_as_real(k)).all()
+        assert _rms(k, out[0]) < 1e-6
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("kw", [dict(), dict(stokes_ids=(1, 2, 3, 4)), dict(sup=11)], ids=["i", "iquv", "wide"])
+def test_gridding_values_that_are_not_finite(kw, fp64):
+    """A NaN and an Inf reach the cells of their own footprints and no others; rows with NaN coordinates
+    reach none."""
+    c = cases.make_case(seed=64, nant=7, ntimes=10, nchan=8, ncorr=4, npix=127, cell_arcsec=5.0, nw=2, **kw)
+    c.uvw = c.uvw.copy()
+    c.uvw[5, 2] = np.nan
+    c.uvw[9, 0] = np.nan
+    vs, fg, _ = cases._gpu_objs(c)
+    geo = _geometry(c, vs, fg)
+    assert (geo[5, :, 0] != 1).all() and (geo[9, :, 0] != 1).all()
+    pick = [(r, ch) for r, ch in ((40, 2), (90, 5)) if geo[r, ch, 0] == 1]
+    assert len(pick) == 2
+    vs.vis[pick[0]] = complex(float("nan"), 0.0)
+    vs.vis[pick[1]] = complex(float("inf"), 0.0)
+    want = np.ones((c.npix, c.npix), bool)
+    for r, ch in pick:
+        sup = int(fg.cf.sup[geo[r, ch, 2]])
+        x, y = geo[r, ch, 3] - (sup - 1) // 2, geo[r, ch, 4] - (sup - 1) // 2
+        want[y:y + sup, x:x + sup] = False
+    g = dataclasses.replace(fg, grid=torch.zeros_like(fg.grid), grid_acc=None)
+    if fp64:
+        g.with_fp64_accumulation()
+    D.grid(vs, [g], D.make_pol(c.corr_ids, c.stokes_ids), batch=D.Batch.create())
+    ok = torch.isfinite(torch.view_as_real(g.grid)).all(-1).cpu().numpy()
+    for p in range(c.npol):
+        assert np.array_equal(ok[0, p], want)
+    if fp64:
+        assert torch.count_nonzero(torch.view_as_real(g.grid_acc)) == 0
