@@ -202,8 +202,19 @@ class FacetMachine:
     def _work_for(self, n):
         need = self.nband * self.npol * n * n
         if self._work is None or self._work.numel() < need:
-            self._work = torch.empty(need, dtype=torch.complex64, device=self.device)
+            # for the largest facet at once: a smaller buffer given back here could still be in use on
+            # another stream
+            most = max([n, *(f.grid.grid.shape[-1] for f in self.facets)])
+            self._work = torch.empty(self.nband * self.npol * most * most, dtype=torch.complex64, device=self.device)
         return self._work
+
+    def _zeros(self, m, stream):
+        """A zero image, zeroed on the stream that adds to it (None: the current one)."""
+        with torch.cuda.stream(stream):
+            image = torch.zeros((self.nband, self.npol, m, m), dtype=torch.float32, device=self.device)
+        if stream is not None:
+            image.record_stream(torch.cuda.current_stream())  # where the caller may use it
+        return image
 
     # --------------------------------------------------------------------------------------
     def reset_grids(self):
@@ -227,7 +238,7 @@ class FacetMachine:
         lib = _abi.lib()
         st = D._stream_ptr(stream)
         m = self.npix_out
-        image = torch.zeros((self.nband, self.npol, m, m), dtype=torch.float32, device=self.device)
+        image = self._zeros(m, stream)
         for f in self.facets:
             n = f.grid.grid.shape[-1]
             xc, yc = f.geom.pix_central
@@ -271,7 +282,7 @@ class FacetMachine:
         m = self.npix_out
         if len(grid_grads) != len(self.facets):
             raise ValueError("one grid gradient per facet")
-        grad = torch.zeros((self.nband, self.npol, m, m), dtype=torch.float32, device=self.device)
+        grad = self._zeros(m, stream)
         for f, g in zip(self.facets, grid_grads):
             if g is None:
                 continue

@@ -141,3 +141,31 @@ def test_gridding_values_that_are_not_finite(kw, fp64):
         assert np.array_equal(ok[0, p], want)
     if fp64:
         assert torch.count_nonzero(torch.view_as_real(g.grid_acc)) == 0
+
+
+def test_images_on_a_stream_of_the_callers():
+    """The image is zeroed on the stream that adds to it, however busy the current one is."""
+    from ddfacet_b200.facetmachine import FacetMachine
+
+    fm = FacetMachine(300, 6.0, 2, np.linspace(1.3e9, 1.45e9, 4), nw=2, wmax=500.0)
+    for i, f in enumerate(fm.facets):
+        f.grid.sumwt.fill_(3.0)
+        f.model.grid.copy_(_randn(f.model.grid.shape, 20 + i))
+    grids = [_randn(f.grid.grid.shape, i) for i, f in enumerate(fm.facets)]
+    grads = [f.model.grid for f in fm.facets]
+
+    def images(stream):
+        for f, g in zip(fm.facets, grids):
+            f.grid.grid.copy_(g)
+        torch.cuda.synchronize()
+        if stream is not None:
+            torch.cuda._sleep(200_000_000)  # a tenth of a second
+        out = fm.facets_to_image(stream=stream), fm.image_to_facets_adjoint(grads, stream=stream)
+        torch.cuda.synchronize()
+        return out
+
+    want = images(None)
+    got = images(torch.cuda.Stream())
+    for a, b in zip(got, want):
+        assert torch.count_nonzero(b) > 0
+        assert torch.equal(a, b)
