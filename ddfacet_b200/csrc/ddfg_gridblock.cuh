@@ -382,10 +382,10 @@ __device__ __forceinline__ void warp_add_single_sums(const ddfg_vis &vs, const d
         a_sumj[f.nband + g] += (double)npol_used * wsum;
       }
     }
-    __syncwarp();
   } else {
     warp_add_sums<NPOL>(js, f, rec, npol_used, a_sumwt, a_sumj);
   }
+  __syncwarp();  // the next stripe's sums may be another lane's, plain or atomic
   if (js.mode != 0 && rec.valid && f.sumjones_chan) {
     const double j = (double)npol_used * rec.sumjones, q = (double)npol_used * rec.sumsqw;
     if (s_chan) {

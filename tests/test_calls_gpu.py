@@ -169,3 +169,20 @@ def test_images_on_a_stream_of_the_callers():
     for a, b in zip(got, want):
         assert torch.count_nonzero(b) > 0
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("nch", [0, 1, 6])
+def test_sums_of_stripes_with_one_band_and_two(nch):
+    """96 channels in two bands of 48: of a row's three stripes the outer two add up in one lane and the
+    middle one with atomics, to the same slots.  FP64 sums of FP32 weights: 1e-12, times FP32 Jones
+    weights: 1e-6."""
+    c = cases.make_case(seed=66, nant=10, ntimes=20, nchan=96, ncorr=4, npix=127, cell_arcsec=5.0, nw=2, nband=2,
+                        flag_frac=0.05)
+    if nch:
+        cases.add_jones(c, nt=2, nd=2, mode=1, nch=nch)
+    want = cases.run_fp64_grid(c)
+    got = cases.run_gpu_grid(c, batched=True)
+    np.testing.assert_allclose(got["sumwt"], want["sumwt"], rtol=1e-12)
+    if nch:
+        np.testing.assert_allclose(got["sumjones"], want["sumjones"], rtol=1e-6)
+        np.testing.assert_allclose(got["sumjones_chan"], want["sumjones_chan"], rtol=1e-6)
