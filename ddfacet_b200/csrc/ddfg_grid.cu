@@ -67,9 +67,9 @@ __device__ __forceinline__ void flush_grid_sums(const ddfg_facet *sf, int npk, c
 
 // Single-visibility blocks: each warp loads its 32 visibilities' facet-independent inputs (map
 // entries, uvw, flags, weights, visibilities, Jones indices) once and grids them onto every facet
-// of the pack in turn.
-template <int NPOL, int SLOTS>
-__global__ void __launch_bounds__(256) grid_single_q(const ddfg_vis vs, const ddfg_jones js,
+// of the pack in turn.  ACC: facets may have FP64 accumulators.
+template <int NPOL, int SLOTS, bool ACC>
+__global__ void __launch_bounds__(256, NPOL == 2 && SLOTS == 4 ? 1 : 2) grid_single_q(const ddfg_vis vs, const ddfg_jones js,
                                                      const __grid_constant__ FacetTable tab, const GridParams gp,
                                                      const Sched sc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) grid_single_q(const ddfg_vis vs, const dd
           grid_single_facet<NPOL>(in, vs, js, f, gp, s_n0m1[fi], rec);
           warp_add_single_sums<NPOL>(vs, js, f, rec, npol_used, all, one_band, wsum, a, a + f.nband * f.npol,
                                      sc.chan_sums ? a + (nwarps - warp) * sc.small_stride : nullptr);
-          scatter<NPOL, SLOTS>(rec, f, npol_used, ws, lane);
+          scatter<NPOL, SLOTS, false, false, ACC>(rec, f, npol_used, ws, lane);
         }
       }
     }
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) grid_single_i(const ddfg_vis vs, const dd
 // facets.  A large-block item gives its block to the whole warp: lane 0 walks the FP64 means in the
 // reference's order, the warp the rest (grid_block_record_warp).  The block walk needs ~170
 // registers: CTAs of 128 threads, three per SM.
-template <int NPOL, int SLOTS>
+template <int NPOL, int SLOTS, bool ACC>
 __global__ void __launch_bounds__(128, 3) grid_block_q(const ddfg_vis vs, const ddfg_jones js,
                                                        const __grid_constant__ FacetTable tab, const GridParams gp,
                                                        const Sched sc) {
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(128, 3) grid_block_q(const ddfg_vis vs, const 
           }
           warp_add_block_sums<NPOL>(vs, js, f, gp, b, rec, npol_used, a, a + f.nband * f.npol, a_chan, jc,
                                     large && !rec.single_chan);
-          scatter<NPOL, SLOTS, false, true>(rec, f, npol_used, ws, lane);
+          scatter<NPOL, SLOTS, false, true, ACC>(rec, f, npol_used, ws, lane);
         }
       }
     }
@@ -453,13 +453,15 @@ size_t grid_facet_smem(int warps, int acc_stride, bool stokes_i, bool single) {
 
 template <int NP, int SL>
 int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable &tab, const GridParams &gp,
-                      Sched sc, const ddfg_batch *batch, bool &zeroed, int counters, cudaStream_t stream) {
+                      Sched sc, const ddfg_batch *batch, bool acc, bool &zeroed, int counters, cudaStream_t stream) {
   const bool single = vs->single_vis_blocks != 0, stokes_i = NP == 1 && grid_is_i(vs, js, gp);
   const int threads = single ? 256 : 128;
   const size_t smem = grid_smem<NP, SL>(threads / 32) +
                       (size_t)sc.max_pack * grid_facet_smem(threads / 32, sc.acc_stride, stokes_i, single);
+  constexpr bool one = NP == 1;  // one plane: one kernel for both kinds of grid
   const void *kern = stokes_i ? (single ? (const void *)grid_single_i<SL> : (const void *)grid_block_i<SL>)
-                              : (single ? (const void *)grid_single_q<NP, SL> : (const void *)grid_block_q<NP, SL>);
+                     : acc ? (single ? (const void *)grid_single_q<NP, SL, true> : (const void *)grid_block_q<NP, SL, true>)
+                           : (single ? (const void *)grid_single_q<NP, SL, one> : (const void *)grid_block_q<NP, SL, one>);
   int per_sm = 0;
   int rc = ddfg_kernel_prepare(kern, threads, smem, &per_sm);
   if (rc) return rc;
@@ -469,8 +471,10 @@ int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable
   if ((rc = sched_counters(sc, false, ctas * (threads / 32), zeroed, counters, stream))) return rc;
   if (stokes_i && single) grid_single_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (stokes_i) grid_block_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
-  else if (single) grid_single_q<NP, SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
-  else grid_block_q<NP, SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
+  else if (single && acc) grid_single_q<NP, SL, true><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
+  else if (single) grid_single_q<NP, SL, one><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
+  else if (acc) grid_block_q<NP, SL, true><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
+  else grid_block_q<NP, SL, one><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ddfg_set_error(DDFG_ECUDA, "grid launch: %s", cudaGetErrorString(e));
   return DDFG_OK;
@@ -532,7 +536,7 @@ int ddfg_launch_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet 
     sc.large_items = nlarge;
     sc.counter = counters ? counters + f0 : nullptr;  // a launch has at most as many packs as facets
     int rc;
-#define LG(NP, SL) rc = launch_grid_table<NP, SL>(vs, js, tab_tl, gp, sc, batch, zeroed, nfacets - f0, stream)
+#define LG(NP, SL) rc = launch_grid_table<NP, SL>(vs, js, tab_tl, gp, sc, batch, any_acc, zeroed, nfacets - f0, stream)
     if (slots == 2) {
       switch (nvispol) {
         case 1: LG(1, 2); break;

@@ -91,15 +91,18 @@ __device__ __forceinline__ void red_add_f64(double *p, double v) {
 // 2i+1 swap halves so that each reduction carries whole cells.  A cell's two doubles in one
 // instruction are one sector operation instead of two, and the sectors are what FP64 reductions
 // cost: 7 x 7 footprints, 249 G cells/s against 126 G cells/s with one instruction for the real and
-// one for the imaginary parts.
-__device__ __forceinline__ void red_add_cells_f64(double *acc, int cell, float2 v, int lane) {
+// one for the imaginary parts.  Cells ca and cb are the pair's first and second.
+template <typename T2>
+__device__ __forceinline__ void red_add_pair_f64(double *acc, int ca, int cb, T2 v, int lane) {
   const bool odd = lane & 1;
-  const float got = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
-  const int other = __shfl_xor_sync(0xffffffffu, cell, 1);
-  const int ca = odd ? other : cell, cb = odd ? cell : other;
+  const auto got = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
   double *d = acc + (lane & 1);
   if (ca >= 0) red_add_f64(d + 2 * (size_t)ca, odd ? got : v.x);
   if (cb >= 0) red_add_f64(d + 2 * (size_t)cb, odd ? v.y : got);
+}
+__device__ __forceinline__ void red_add_cells_f64(double *acc, int cell, float2 v, int lane) {
+  const int other = __shfl_xor_sync(0xffffffffu, cell, 1);
+  red_add_pair_f64(acc, lane & 1 ? other : cell, lane & 1 ? cell : other, v, lane);
 }
 
 // Adds the products of n records (a multiple of four) of support S to the tile, taps first ..
@@ -213,8 +216,9 @@ __device__ __forceinline__ void tile_to_grid(unsigned tile, int bw, int bh, int 
 // channels up to 12 cells apart, with the window below: 32 us to 22 us).
 constexpr int kFewRecords = 2;
 
-// BLOCKS: averaged blocks, whose runs are long (0.1 cells a block) -- an FP64 accumulator gets FP64
-// runs; single visibilities' runs of about three are summed in FP32 as they always were.
+// A run on its way to an FP64 accumulator: averaged blocks' runs are long (0.1 cells a block) and are summed
+// in FP64; single visibilities of one support up to 16 have runs of about three, whose sum in FP32 loses
+// less than the products' own roundings; those of wide or mixed supports take no runs.
 template <int SLOTS, bool CONJ, bool BLOCKS, int CELLS>
 __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddfg_facet &f, TileSmem<CELLS> &sm,
                                              int lane) {
@@ -223,12 +227,14 @@ __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddf
   static_assert(W * W <= CELLS, "tile");
   unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
   const int bx = rec.g.locx - rec.g.sup, by = rec.g.locy - rec.g.sup;
+  unsigned other = 0;  // records of another support or band
   while (mask) {
     // the records of one support and band that the tile covers together
     const int lead = __ffs(mask) - 1;
     const int S = __shfl_sync(0xffffffffu, rec.g.S, lead), band = __shfl_sync(0xffffffffu, rec.gridchan, lead);
     const bool like = (mask >> lane & 1) && rec.g.S == S && rec.gridchan == band;
     unsigned seg = __ballot_sync(0xffffffffu, like);
+    other |= seg ^ mask;
     int x0 = __reduce_min_sync(0xffffffffu, like ? bx : 0x7fffffff);
     int y0 = __reduce_min_sync(0xffffffffu, like ? by : 0x7fffffff);
     int bw = __reduce_max_sync(0xffffffffu, like ? bx : -1) - x0 + S;
@@ -284,8 +290,9 @@ __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddf
         for (int j = n; j < n4; ++j) sm.rec[j] = make_int4(to, rec.g.cfoff, 0, 0);
     }
     __syncwarp();
-    const unsigned runs =
+    unsigned runs =
         __ballot_sync(0xffffffffu, lane > 0 && lane < n && sm.rec[lane].x != sm.rec[lane > 0 ? lane - 1 : 0].x);
+    if (!BLOCKS && ((SLOTS > 2 && S > 16) || other) && f64) runs = 0xffffffffu;  // no runs: into the FP64 tile
     const int step = SLOTS == 2 || S <= 8 ? 64 : 32 * SLOTS;
     for (int first = 0; first < S * S; first += step) {
       if (SLOTS == 2 || S <= 8) {
@@ -308,7 +315,7 @@ __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddf
 // exactly one cell (x, y) has (y mod S) S + (x mod S) = t, so the lane's cell for the next record is
 // the same one as long as the window still covers it.  The lane keeps adding into registers and
 // reaches memory only when the window leaves its cell: a move by one column costs S additions a
-// plane, not S^2.  (A facet with an FP64 accumulator still takes every run.)
+// plane, not S^2.
 
 // x mod S for 0 <= x < 2^26, magic = torus_magic(S).
 __device__ __forceinline__ unsigned torus_magic(int S) { return 0xffffffffu / (unsigned)S + 1u; }
@@ -355,12 +362,11 @@ struct alignas(16) TorusSmem {
   float2 st[NPOL > 1 ? NPOL - 1 : 1][32];
 };
 
-// One pass of the torus over n records (n a multiple of four) of support S.
+// One pass of the torus over n records (n a multiple of four) of support S, into the float32 grid.
 template <int NPOL, int SLOTS, bool CONJ>
 __device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int S, int first,
-                                             const ddfg_facet &f, int npol_used, int lane) {
+                                           const ddfg_facet &f, int npol_used, int lane) {
   float2 *const grid = (float2 *)f.grid;
-  double *const acc64 = (double *)f.grid_acc;
   const float2 *const cfd = (const float2 *)f.cf_data;
   const int nx = f.nx;
   const size_t plane = (size_t)f.nx * f.ny;
@@ -378,8 +384,7 @@ __device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int
 #pragma unroll
     for (int p = 0; p < NPOL; ++p) {
       if (p >= npol_used) break;
-      if (acc64) red_add_cells_f64(acc64 + 2 * p * plane, to, a[p][k], lane);
-      else if (to >= 0) red_add(grid + p * plane + to, a[p][k]);
+      if (to >= 0) red_add(grid + p * plane + to, a[p][k]);
     }
   };
   int cur = -1, ahead = -1;  // origin of the sums, origin of the records being loaded
@@ -406,9 +411,8 @@ __device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int
         cur = q[r].x;
 #pragma unroll
         for (int k = 0; k < SLOTS; ++k) {
-          // FP64 sums take every run by itself, as FP64 additions did before runs merged
-          const bool leave = acc64 || to[r][k] != cell[k];
-          flush(k, leave ? cell[k] : -1);
+          const bool leave = to[r][k] != cell[k];
+          flush(k, leave ? cell[k] : -1);  // not inside the branch: 1.55 ms instead of 1.25
           if (leave) {
             cell[k] = to[r][k];
 #pragma unroll
@@ -429,17 +433,100 @@ __device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int
   for (int k = 0; k < SLOTS; ++k) flush(k, cell[k]);
 }
 
+// All passes over n records of support S into the facet's FP64 accumulator, which takes every run by
+// itself.  RUN64: the run's FP32 products are summed in FP64.  A record at a time (its successor's taps in
+// flight) and out of line: with four at once, as in torus_pass, the additions of eight cells stand in the
+// code four times, and the kernel waits for its instructions (four planes, supports up to 23, FP64 runs:
+// 15.8 ms, 5.2 ms this way; with both kinds of grid in one loop the float32 one takes 2.47 ms instead of
+// 1.25).
+template <int NPOL, bool RUN64>
+__device__ __noinline__ void torus_acc(const TorusSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, int npol_used,
+                                       int lane) {
+  using Sum = typename std::conditional<RUN64, double2, float2>::type;
+  double *const acc = (double *)f.grid_acc;
+  const float2 *const cfd = (const float2 *)f.cf_data;
+  const int nx = f.nx;
+  const size_t plane = (size_t)f.nx * f.ny;
+  for (int first = 0; first < S * S; first += 64) {
+    TorusLane<2> tl;
+    tl.set(S, first + lane);
+    int cell[2] = {-1, -1}, to[2];
+    Sum a[NPOL][2];
+    float2 c[2];
+    int cur = -1, ahead = -1;
+    auto load = [&](int i) {
+      const int4 q = sm.rec[i];
+      if (q.x != ahead) {  // the same for all lanes
+        ahead = q.x;
+        tl.move(ahead, sm.mod[i], S, nx);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        to[k] = tl.cell[k];
+        c[k] = __ldg(cfd + (q.y + tl.off[k]));
+      }
+    };
+    auto flush = [&]() {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int other = __shfl_xor_sync(0xffffffffu, cell[k], 1);
+        const int ca = lane & 1 ? other : cell[k], cb = lane & 1 ? cell[k] : other;
+#pragma unroll
+        for (int p = 0; p < NPOL; ++p) {
+          if (p >= npol_used) break;
+          red_add_pair_f64(acc + 2 * p * plane, ca, cb, a[p][k], lane);
+        }
+      }
+    };
+    load(0);
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const int4 q = sm.rec[i];
+      const float2 tap[2] = {c[0], c[1]};
+      const int at[2] = {to[0], to[1]};
+      if (i + 1 < n) load(i + 1);
+      if (q.x != cur) {
+        if (cur >= 0) flush();
+        cur = q.x;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          cell[k] = at[k];
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p) a[p][k].x = a[p][k].y = 0;
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < NPOL; ++p) {
+        const float2 v = p == 0 ? make_float2(__int_as_float(q.z), __int_as_float(q.w)) : sm.st[p > 0 ? p - 1 : 0][i];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if constexpr (RUN64) {
+            const float2 t = cmul(tap[k], v);
+            a[p][k].x += (double)t.x;
+            a[p][k].y += (double)t.y;
+          } else {
+            a[p][k] = cfma(tap[k], v, a[p][k]);
+          }
+        }
+      }
+    }
+    flush();
+  }
+}
+
 // Adds the warp's 32 records to facet f (gridder.h:353-362): into the FP64 accumulator when the
 // facet has one, else into the float32 grid.  CONJ lays down conj(CF) (the adjoint of the
 // degridder's gather).  sm: the warp's own.  Must be called by all 32 lanes.
-template <int NPOL, int SLOTS, bool CONJ = false>
+template <int NPOL, int SLOTS, bool CONJ, bool BLOCKS, bool ACC>
 __device__ __forceinline__ void scatter_torus(const GridRecord<NPOL> &rec, const ddfg_facet &f, int npol_used,
                                               TorusSmem<NPOL> &sm, int lane) {
   unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
+  bool mixed = false;  // several supports
   while (mask) {
     const int S = __shfl_sync(0xffffffffu, rec.g.S, __ffs(mask) - 1);
     const bool mine = rec.valid && rec.g.S == S;
     const unsigned sub = __ballot_sync(0xffffffffu, mine);
+    mixed = mixed || sub != mask;
     mask &= ~sub;
     const int n = __popc(sub), n4 = (n + 3) & ~3;
     int base = 0, mod = 0, cfo = 0;
@@ -467,7 +554,10 @@ __device__ __forceinline__ void scatter_torus(const GridRecord<NPOL> &rec, const
       for (int p = 1; p < NPOL; ++p) sm.st[p > 0 ? p - 1 : 0][n + lane] = czero();
     }
     __syncwarp();
-    if (SLOTS > 2 && S <= 8) {
+    if (ACC && f.grid_acc) {
+      if (BLOCKS || S > 16 || mixed) torus_acc<NPOL, true>(sm, n, S, f, npol_used, lane);
+      else torus_acc<NPOL, false>(sm, n, S, f, npol_used, lane);
+    } else if (SLOTS > 2 && S <= 8) {
       torus_pass<NPOL, 2, CONJ>(sm, n4, S, 0, f, npol_used, lane);
     } else {
       for (int first = 0; first < S * S; first += 32 * SLOTS)
@@ -494,12 +584,13 @@ struct ScatterSmem<1, SLOTS> {
   }
 };
 
-// The warp's records onto facet f.  sm: the warp's own, cleared once (clear) before the first call.
-template <int NPOL, int SLOTS, bool CONJ = false, bool BLOCKS = false>
+// The warp's records onto facet f.  sm: the warp's own, cleared once (clear) before the first call.  ACC:
+// facets may have FP64 accumulators (several planes only, where that code costs the other path registers).
+template <int NPOL, int SLOTS, bool CONJ = false, bool BLOCKS = false, bool ACC = !CONJ>
 __device__ __forceinline__ void scatter(const GridRecord<NPOL> &rec, const ddfg_facet &f, int npol_used,
                                         ScatterSmem<NPOL, SLOTS> &sm, int lane) {
   if constexpr (NPOL == 1) scatter_tile<SLOTS, CONJ, BLOCKS>(rec, f, sm.tile, lane);
-  else scatter_torus<NPOL, SLOTS, CONJ>(rec, f, npol_used, sm.torus, lane);
+  else scatter_torus<NPOL, SLOTS, CONJ, BLOCKS, ACC>(rec, f, npol_used, sm.torus, lane);
 }
 
 // ----------------------------------------------------------------------------------------

@@ -209,3 +209,29 @@ def test_long_blocks_of_coherent_visibilities():
     vs, fg, _ = cases._gpu_objs(c)
     assert vs.nblocks == 10 and not vs.single_vis_blocks
     assert _grid_error(c, vs, fg) < 1e-7
+
+
+@pytest.mark.parametrize("kw", [dict(sup=17), dict(sup=23), dict(sup=19, stokes_ids=(1, 2, 3, 4)),
+                                dict(sup=7, stokes_ids=(1, 2, 3, 4), blocks=True),
+                                dict(sup=11, stokes_ids=(1, 2), blocks=True), dict(sup=7, blocks=True)],
+                         ids=["i17", "i23", "iquv19", "iquv_blocks", "iq11_blocks", "i_blocks"])
+def test_runs_reach_the_accumulator_in_fp64(kw):
+    """One baseline's 32 channels on one cell, FP64 sums: the products add up in FP64 where supports are
+    wide or blocks averaged.  Of a cell's own value, RMS over the cells: the cell's rounding at the end
+    2.6e-8, those of 32 products (3.5e-8 each, independent) and of the 32 values 6e-9 each: 2.8e-8, with
+    room to 4e-8; a sum of 32 in FP32 has 8e-8."""
+    kw = dict(kw)
+    blocks = kw.pop("blocks", False)
+    c = _coherent(2, 2 if blocks else 1, f_lo=1.4e9, f_hi=1.4001e9, **kw)
+    if blocks:  # the second row in one block, which makes the map an averaged one; it is flagged
+        blk = [[ch, ch + 1, 0] for ch in range(c.nchan)] + [[0, c.nchan, 1]]
+        c.bda = np.concatenate([bda._header(len(blk)), [len(b) for b in blk], *blk]).astype(np.int32)
+        c.flags[1] = True
+    vs, fg, _ = cases._gpu_objs(c)
+    assert bool(vs.single_vis_blocks) != blocks
+    g = dataclasses.replace(fg, grid=torch.zeros_like(fg.grid)).with_fp64_accumulation()
+    D.grid(vs, [g], D.make_pol(c.corr_ids, c.stokes_ids), batch=D.Batch.create())
+    want = cases.run_fp64_grid(c)["grid"]
+    on = want != 0
+    got = g.grid.cpu().numpy().astype(np.complex128)[on]
+    assert np.sqrt(np.mean(np.abs(got / want[on] - 1) ** 2)) < 4e-8
