@@ -40,21 +40,20 @@
 
 namespace ddfg {
 
-// Adds the CTA's shared sums of the pack's npk facets to their float64 outputs.  Each facet's
-// accumulators are one copy of the weight and Jones sums per warp (updated by that warp alone, so
-// its lanes never contend with other warps for them), then the per-channel Jones sums (chan_sums).
+constexpr int kBlockWarps = 12;  // warps an SM of the averaged-block kernels
+
+// Adds the CTA's shared sums of the pack's npk facets to their float64 outputs.
 __device__ __forceinline__ void flush_grid_sums(const ddfg_facet *sf, int npk, const double *s_acc, const Sched &sc,
                                                 const ddfg_jones &js, int nchan) {
-  const int nwarps = blockDim.x >> 5;
   for (int fi = 0; fi < npk; ++fi) {
     const ddfg_facet &f = sf[fi];
     const double *a = s_acc + (size_t)fi * sc.acc_stride;
-    const double *a_chan = a + nwarps * sc.small_stride;
+    const double *a_chan = a + sc.small_copies * sc.small_stride;
     const int nsw = f.nband * f.npol;
     const int nsmall = nsw + (js.mode != 0 ? 2 * f.nband : 0);
     for (int i = threadIdx.x; i < nsmall; i += blockDim.x) {
       double v = 0.;
-      for (int w = 0; w < nwarps; ++w) v += a[w * sc.small_stride + i];
+      for (int w = 0; w < sc.small_copies; ++w) v += a[w * sc.small_stride + i];
       double *dst = i < nsw ? f.sumwt + i : (f.sumjones ? f.sumjones + (i - nsw) : nullptr);
       if (i < nsw && !f.sumwt) dst = nullptr;
       if (dst && v != 0.) atomicAdd(dst, v);
@@ -103,11 +102,12 @@ __global__ void __launch_bounds__(256, NPOL == 2 && SLOTS == 4 ? 1 : 2) grid_sin
         for (int fi = 0; fi < npk; ++fi) {
           const ddfg_facet &f = sf[fi];
           const int npol_used = min(gp.nvispol, f.npol);
-          double *a = s_acc + (size_t)fi * sc.acc_stride + warp * sc.small_stride;  // this warp's sums
+          double *acc = s_acc + (size_t)fi * sc.acc_stride, *a = acc + warp * sc.warp_stride;  // this warp's sums
           GridRecord<NPOL> rec;
           grid_single_facet<NPOL>(in, vs, js, f, gp, s_n0m1[fi], rec);
-          warp_add_single_sums<NPOL>(vs, js, f, rec, npol_used, all, one_band, wsum, a, a + f.nband * f.npol,
-                                     sc.chan_sums ? a + (nwarps - warp) * sc.small_stride : nullptr);
+          warp_add_single_sums<NPOL>(vs, js, f, rec, npol_used, all, one_band, wsum, sc.warp_stride != 0, a,
+                                     a + f.nband * f.npol,
+                                     sc.chan_sums ? acc + sc.small_copies * sc.small_stride : nullptr);
           scatter<NPOL, SLOTS, false, false, ACC>(rec, f, npol_used, ws, lane);
         }
       }
@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(256, NPOL == 2 && SLOTS == 4 ? 1 : 2) grid_sin
 }
 
 // The same for Stokes I from the diagonal correlations, without smearing and with Jones terms as
-// stored (ddfg_single.cuh).
-template <int SLOTS>
+// stored (ddfg_single.cuh).  BANDS: facets have several bands.
+template <int SLOTS, bool BANDS>
 __global__ void __launch_bounds__(256) grid_single_i(const ddfg_vis vs, const ddfg_jones js,
                                                      const __grid_constant__ FacetTable tab, const GridParams gp,
                                                      const Sched sc) {
@@ -179,10 +179,11 @@ __global__ void __launch_bounds__(256) grid_single_i(const ddfg_vis vs, const dd
           rec.sumjones = (double)rec.bb * in.fw;
           rec.ch0 = in.ch;
           rec.single_chan = true;
-          double *a = s_acc + (size_t)fi * sc.acc_stride + warp * sc.small_stride;  // this warp's sums
-          warp_add_single_sums<1>(vs, js, sf[fi], rec, 1, all, one_band, wsum, a, a + f.nband * f.npol,
-                                  sc.chan_sums ? a + (nwarps - warp) * sc.small_stride : nullptr);
-          scatter<1, SLOTS>(rec, sf[fi], 1, ws, lane);
+          double *acc = s_acc + (size_t)fi * sc.acc_stride, *a = acc + warp * sc.warp_stride;  // this warp's sums
+          warp_add_single_sums<1>(vs, js, sf[fi], rec, 1, all, one_band, wsum, sc.warp_stride != 0, a,
+                                  a + f.nband * f.npol,
+                                  sc.chan_sums ? acc + sc.small_copies * sc.small_stride : nullptr);
+          scatter<1, SLOTS, false, false, true, BANDS>(rec, sf[fi], 1, ws, lane);
         }
       }
     }
@@ -196,9 +197,9 @@ __global__ void __launch_bounds__(256) grid_single_i(const ddfg_vis vs, const dd
 // visibilities, flags and weights come from DRAM once per pack and from L1/L2 for the other
 // facets.  A large-block item gives its block to the whole warp: lane 0 walks the FP64 means in the
 // reference's order, the warp the rest (grid_block_record_warp).  The block walk needs ~170
-// registers: CTAs of 128 threads, three per SM.
+// registers: twelve warps an SM, as three CTAs of four or (where one facet's sums need it) one of twelve.
 template <int NPOL, int SLOTS, bool ACC>
-__global__ void __launch_bounds__(128, 3) grid_block_q(const ddfg_vis vs, const ddfg_jones js,
+__global__ void __launch_bounds__(kBlockWarps * 32, 1) grid_block_q(const ddfg_vis vs, const ddfg_jones js,
                                                        const __grid_constant__ FacetTable tab, const GridParams gp,
                                                        const Sched sc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -235,8 +236,8 @@ __global__ void __launch_bounds__(128, 3) grid_block_q(const ddfg_vis vs, const 
         for (int fi = 0; fi < npk; ++fi) {
           const ddfg_facet &f = sf[fi];
           const int npol_used = min(gp.nvispol, f.npol);
-          double *a = s_acc + (size_t)fi * sc.acc_stride + warp * sc.small_stride;
-          double *a_chan = s_acc + (size_t)fi * sc.acc_stride + (blockDim.x >> 5) * sc.small_stride;
+          double *acc = s_acc + (size_t)fi * sc.acc_stride, *a = acc + warp * sc.warp_stride;
+          double *a_chan = acc + sc.small_copies * sc.small_stride;
           GridRecord<NPOL> rec;
           rec.valid = false;
           rec.single_chan = true;
@@ -319,7 +320,7 @@ __device__ __forceinline__ BlockSums block_sums_i(const ddfg_vis &vs, const ddfg
 // walk).  One third of grid_block_q's code: that kernel ran at 0.9 instructions a cycle and SM on
 // averaged blocks, waiting for instructions most of the time.
 template <int SLOTS>
-__global__ void __launch_bounds__(128, 3) grid_block_i(const ddfg_vis vs, const ddfg_jones js,
+__global__ void __launch_bounds__(kBlockWarps * 32, 1) grid_block_i(const ddfg_vis vs, const ddfg_jones js,
                                                        const __grid_constant__ FacetTable tab, const GridParams gp,
                                                        const Sched sc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -365,8 +366,8 @@ __global__ void __launch_bounds__(128, 3) grid_block_i(const ddfg_vis vs, const 
           const FacetI &f = sfi[fi];
           if (large && (fi & 31) == 0 && fi + lane < npk)
             lm = block_means_i(vs, sfi[fi + lane].cu, sfi[fi + lane].cv, r.rows, r.nrows, r.ch0, r.ch1);
-          double *a = s_acc + (size_t)fi * sc.acc_stride + warp * sc.small_stride;  // this warp's sums
-          double *s_chan = sf[fi].sumjones_chan ? a + (nwarps - warp) * sc.small_stride : nullptr;
+          double *acc = s_acc + (size_t)fi * sc.acc_stride, *a = acc + warp * sc.warp_stride;  // this warp's sums
+          double *s_chan = sf[fi].sumjones_chan ? acc + sc.small_copies * sc.small_stride : nullptr;
           GridRecord<1> rec;
           rec.valid = false;
           BlockMeans m;
@@ -453,13 +454,17 @@ size_t grid_facet_smem(int warps, int acc_stride, bool stokes_i, bool single) {
 
 template <int NP, int SL>
 int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable &tab, const GridParams &gp,
-                      Sched sc, const ddfg_batch *batch, bool acc, bool &zeroed, int counters, cudaStream_t stream) {
+                      Sched sc, int threads, const ddfg_batch *batch, bool acc, bool &zeroed, int counters,
+                      cudaStream_t stream) {
   const bool single = vs->single_vis_blocks != 0, stokes_i = NP == 1 && grid_is_i(vs, js, gp);
-  const int threads = single ? 256 : 128;
   const size_t smem = grid_smem<NP, SL>(threads / 32) +
                       (size_t)sc.max_pack * grid_facet_smem(threads / 32, sc.acc_stride, stokes_i, single);
   constexpr bool one = NP == 1;  // one plane: one kernel for both kinds of grid
-  const void *kern = stokes_i ? (single ? (const void *)grid_single_i<SL> : (const void *)grid_block_i<SL>)
+  bool bands = false;
+  for (int i = 0; i < sc.nfacets; ++i) bands = bands || tab.f[i].nband > 1;
+  const void *kern = stokes_i ? (!single ? (const void *)grid_block_i<SL>
+                                 : bands ? (const void *)grid_single_i<SL, true>
+                                         : (const void *)grid_single_i<SL, false>)
                      : acc ? (single ? (const void *)grid_single_q<NP, SL, true> : (const void *)grid_block_q<NP, SL, true>)
                            : (single ? (const void *)grid_single_q<NP, SL, one> : (const void *)grid_block_q<NP, SL, one>);
   int per_sm = 0;
@@ -469,7 +474,8 @@ int launch_grid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable
   const int ctas = ddfg_num_ctas(per_sm);
   sched_split(sc, batch, ctas, threads / 32, !single);
   if ((rc = sched_counters(sc, false, ctas * (threads / 32), zeroed, counters, stream))) return rc;
-  if (stokes_i && single) grid_single_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
+  if (stokes_i && single && bands) grid_single_i<SL, true><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
+  else if (stokes_i && single) grid_single_i<SL, false><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (stokes_i) grid_block_i<SL><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (single && acc) grid_single_q<NP, SL, true><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
   else if (single) grid_single_q<NP, SL, one><<<ctas, threads, smem, stream>>>(*vs, *js, tab, gp, sc);
@@ -497,24 +503,42 @@ int ddfg_launch_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet 
   gp.nvispol = nvispol;
   gp.dopsf = dopsf;
   gp.freq_mean0 = vs->freq_mean;
-  const int nwarps_cta = vs->single_vis_blocks ? 8 : 4;
-  const bool single = vs->single_vis_blocks != 0;
-  const bool chan_sums = !single || vs->nchan <= kSharedChannels;
-  const int acc_stride = nwarps_cta * max_band + (chan_sums ? 2 * vs->nchan : 0);
-  const size_t per_facet_smem = grid_facet_smem(nwarps_cta, acc_stride, nvispol == 1 && grid_is_i(vs, js, gp), single);
-  // Shared memory per CTA: two 256-thread CTAs (single-visibility maps) or three 128-thread CTAs
-  // (averaged blocks) per SM, each with its warps' tiles and the shared sums of a pack -- or one CTA per
-  // SM where the sums of one facet (hundreds of bands, thousands of channels) need more.
-  const size_t scatter_smem = nvispol == 1   ? (slots == 2 ? grid_smem<1, 2>(nwarps_cta) : grid_smem<1, 4>(nwarps_cta))
-                              : nvispol == 2 ? grid_smem<2, 2>(nwarps_cta)
-                              : nvispol == 3 ? grid_smem<3, 2>(nwarps_cta)
-                                             : grid_smem<4, 2>(nwarps_cta);
-  size_t budget = single ? 110 * 1024 : 74 * 1024;
-  if (budget < scatter_smem + per_facet_smem) budget = 225 * 1024;
-  const int max_fit = budget < scatter_smem + per_facet_smem ? 0 : (int)((budget - scatter_smem) / per_facet_smem);
-  if (max_fit < 1) return ddfg_set_error(DDFG_ESIZE, "grid: too many bands/channels for the shared accumulators");
+  const bool single = vs->single_vis_blocks != 0, stokes_i = nvispol == 1 && grid_is_i(vs, js, gp);
+  const bool chan_sums = js->mode != 0 && (!single || vs->nchan <= kSharedChannels);
+  // A CTA's warps, copies of the weight and Jones sums and shared memory: two CTAs of eight warps an SM
+  // (single visibilities) or three of four (averaged blocks), each with its warps' tiles and the sums of a
+  // pack.  A copy a warp, or one that the warps share (atomics) where that makes fewer packs: with hundreds
+  // of bands.  Where not even one facet's sums fit (averaged blocks of thousands of channels), all of an
+  // SM's shared memory goes to one CTA, with the warps of three or, where their tiles leave too little, of
+  // one.
+  struct Shape {
+    int warps, copies;
+    size_t smem;
+  };
+  const int warps = single ? 8 : 4;
+  const size_t smem = (single ? 110 : 74) * 1024;
+  const Shape shapes[] = {
+      {warps, warps, smem}, {warps, 1, smem}, {single ? warps : kBlockWarps, 1, 225 * 1024}, {warps, 1, 225 * 1024}};
   int want = (batch && batch->facets_per_pack > 0) ? batch->facets_per_pack : 16;
-  want = max(1, min(want, max_fit));
+  want = max(1, min(want, nfacets));
+  const Shape *shape = nullptr;
+  int acc_stride = 0, fit = 0;
+  for (const Shape &sh : shapes) {
+    if (shape && (fit == want || sh.smem > shape->smem || sh.warps < shape->warps)) break;
+    const int stride = sh.copies * max_band + (chan_sums ? 2 * vs->nchan : 0);
+    const size_t per_facet = grid_facet_smem(sh.warps, stride, stokes_i, single);
+    const size_t scatter = nvispol == 1   ? (slots == 2 ? grid_smem<1, 2>(sh.warps) : grid_smem<1, 4>(sh.warps))
+                           : nvispol == 2 ? grid_smem<2, 2>(sh.warps)
+                           : nvispol == 3 ? grid_smem<3, 2>(sh.warps)
+                                          : grid_smem<4, 2>(sh.warps);
+    const int n = sh.smem < scatter ? 0 : (int)min((sh.smem - scatter) / per_facet, (size_t)want);
+    if (n < 1 || (shape && (nfacets + n - 1) / n >= (nfacets + fit - 1) / fit)) continue;
+    shape = &sh;
+    acc_stride = stride;
+    fit = n;
+  }
+  if (!shape) return ddfg_set_error(DDFG_ESIZE, "grid: too many bands/channels for the shared accumulators");
+  want = fit;
   unsigned int *counters = batch && !(batch->flags & 1) ? (unsigned int *)batch->workspace : nullptr;  // one a pack
   bool zeroed = false;
   const int ngroups = (nfacets + DDFG_TABLE_FACETS - 1) / DDFG_TABLE_FACETS;
@@ -531,12 +555,14 @@ int ddfg_launch_grid(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_facet 
     sc.max_pack = (n + sc.npacks - 1) / sc.npacks;
     sc.acc_stride = acc_stride;
     sc.small_stride = max_band;
+    sc.small_copies = shape->copies;
+    sc.warp_stride = shape->copies > 1 ? max_band : 0;
     sc.chan_sums = chan_sums;
     sc.nstripes = nstripes;
     sc.large_items = nlarge;
     sc.counter = counters ? counters + f0 : nullptr;  // a launch has at most as many packs as facets
     int rc;
-#define LG(NP, SL) rc = launch_grid_table<NP, SL>(vs, js, tab_tl, gp, sc, batch, any_acc, zeroed, nfacets - f0, stream)
+#define LG(NP, SL) rc = launch_grid_table<NP, SL>(vs, js, tab_tl, gp, sc, 32 * shape->warps, batch, any_acc, zeroed, nfacets - f0, stream)
     if (slots == 2) {
       switch (nvispol) {
         case 1: LG(1, 2); break;

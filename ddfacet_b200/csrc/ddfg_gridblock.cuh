@@ -360,18 +360,19 @@ __device__ __forceinline__ void warp_add_block_sums(const ddfg_vis &vs, const dd
 // The same for single visibilities.  `all` is the lanes with a visibility and wsum their weights'
 // sum, formed once a stripe: a facet that takes them all, in one band and without smearing, needs no
 // reduction of its own for the weights, and none for the Jones sums while their factor is one
-// number (a row's channels share their Jones terms).  s_chan: the CTA's per-channel Jones sums, or
-// NULL (kSharedChannels).
+// number (a row's channels share their Jones terms).  own: no other warp adds to a_sumwt and a_sumj
+// (with others, atomics).
+// s_chan: the CTA's per-channel Jones sums, or NULL (kSharedChannels).
 template <int NPOL>
 __device__ __forceinline__ void warp_add_single_sums(const ddfg_vis &vs, const ddfg_jones &js, const ddfg_facet &f,
                                                      const GridRecord<NPOL> &rec, int npol_used, unsigned all,
-                                                     bool one_band, double wsum, double *a_sumwt, double *a_sumj,
-                                                     double *s_chan) {
+                                                     bool one_band, double wsum, bool own, double *a_sumwt,
+                                                     double *a_sumj, double *s_chan) {
   const unsigned vmask = __ballot_sync(0xffffffffu, rec.valid);
   if (!vmask) return;
   const int lane = threadIdx.x & 31, lead = __ffs(vmask) - 1;
   const float bb0 = __shfl_sync(0xffffffffu, rec.bb, lead);
-  const bool plain = vmask == all && one_band && !vs.uvw_dt &&
+  const bool plain = own && vmask == all && one_band && !vs.uvw_dt &&
                      (js.mode == 0 || __all_sync(0xffffffffu, !rec.valid || rec.bb == bb0));
   if (plain) {
     if (lane == lead) {

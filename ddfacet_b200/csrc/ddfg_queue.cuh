@@ -28,9 +28,12 @@ struct Sched {
   int nfacets;               // facets of this launch
   int npacks;
   int max_pack;              // most facets in one pack (shared-memory sizing)
-  int acc_stride;            // doubles of one facet's shared accumulators (gridding), 0 otherwise:
-                             // [warps][small_stride] weight/Jones sums, then [2][nchan] channel sums (chan_sums)
-  int small_stride;          // doubles of one warp's weight and Jones sums of one facet
+  // Gridding: a facet's shared accumulators are small_copies copies of its weight and Jones sums (one a
+  // warp, or one that the CTA's warps share), then its per-channel Jones sums.
+  int acc_stride;            // doubles of one facet's accumulators, 0 for the other kernels
+  int small_stride;          // doubles of a copy
+  int small_copies;          // warps of a CTA, or 1
+  int warp_stride;           // doubles from a warp's copy to the next warp's: small_stride, or 0
   int chan_sums;             // 1: the shared accumulators hold the per-channel Jones sums
   long long nstripes;        // stripes of 32 blocks
   int chunk;                 // stripes of a CTA's chunk

@@ -215,11 +215,15 @@ __device__ __forceinline__ void tile_to_grid(unsigned tile, int bw, int bh, int 
 // Segments of up to this many records skip the tile (10,800 visibilities of 8 channels on one facet,
 // channels up to 12 cells apart, with the window below: 32 us to 22 us).
 constexpr int kFewRecords = 2;
+// A stripe of bands with no more than this many records each skips it as a whole (64 channels in as many
+// bands: 1.36 ms band by band, 1.09 ms so).
+constexpr int kFewInBand = 2;
 
 // A run on its way to an FP64 accumulator: averaged blocks' runs are long (0.1 cells a block) and are summed
 // in FP64; single visibilities of one support up to 16 have runs of about three, whose sum in FP32 loses
 // less than the products' own roundings; those of wide or mixed supports take no runs.
-template <int SLOTS, bool CONJ, bool BLOCKS, int CELLS>
+// BANDS: facets may have several bands.
+template <int SLOTS, bool CONJ, bool BLOCKS, bool BANDS, int CELLS>
 __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddfg_facet &f, TileSmem<CELLS> &sm,
                                              int lane) {
   const unsigned tile = smem_addr(sm.tile), recs = smem_addr(sm.rec);
@@ -227,19 +231,33 @@ __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddf
   static_assert(W * W <= CELLS, "tile");
   unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
   const int bx = rec.g.locx - rec.g.sup, by = rec.g.locy - rec.g.sup;
-  unsigned other = 0;  // records of another support or band
+  unsigned other = 0;  // records of another support
   while (mask) {
     // the records of one support and band that the tile covers together
     const int lead = __ffs(mask) - 1;
-    const int S = __shfl_sync(0xffffffffu, rec.g.S, lead), band = __shfl_sync(0xffffffffu, rec.gridchan, lead);
-    const bool like = (mask >> lane & 1) && rec.g.S == S && rec.gridchan == band;
+    const int S = __shfl_sync(0xffffffffu, rec.g.S, lead);
+    const int band = BANDS ? __shfl_sync(0xffffffffu, rec.gridchan, lead) : 0;
+    const bool like = (mask >> lane & 1) && rec.g.S == S && (!BANDS || rec.gridchan == band);
     unsigned seg = __ballot_sync(0xffffffffu, like);
-    other |= seg ^ mask;
+    bool few = false;
+    if (!BLOCKS && !BANDS) {
+      other |= seg ^ mask;
+    } else if (!BLOCKS && seg != mask) {
+      const unsigned same = __ballot_sync(0xffffffffu, (mask >> lane & 1) && rec.g.S == S);
+      other |= same ^ mask;
+      if (same != seg) {
+        const bool in = same >> lane & 1;
+        const int bands = __reduce_max_sync(0xffffffffu, in ? rec.gridchan : -1) -
+                          __reduce_min_sync(0xffffffffu, in ? rec.gridchan : 0x7fffffff) + 1;
+        few = __popc(same) <= kFewInBand * bands;
+        if (few) seg = same;
+      }
+    }
     int x0 = __reduce_min_sync(0xffffffffu, like ? bx : 0x7fffffff);
     int y0 = __reduce_min_sync(0xffffffffu, like ? by : 0x7fffffff);
     int bw = __reduce_max_sync(0xffffffffu, like ? bx : -1) - x0 + S;
     int bh = __reduce_max_sync(0xffffffffu, like ? by : -1) - y0 + S;
-    if (bw * bh > CELLS) {
+    if (!few && bw * bh > CELLS) {
       // not all of them: those in a W x W window that starts a cell behind the first record and
       // opens towards the last one (a baseline's records move one way)
       const int last = 31 - __clz(seg), slack = W - S > 1 ? 1 : 0;
@@ -256,14 +274,15 @@ __device__ __forceinline__ void scatter_tile(const GridRecord<1> &rec, const ddf
     }
     mask &= ~seg;
     const float2 *const cfd = (const float2 *)f.cf_data;
-    if (bw * bh > CELLS || (!BLOCKS && __popc(seg) <= kFewRecords)) {
+    if (few || bw * bh > CELLS || (!BLOCKS && __popc(seg) <= kFewRecords)) {
       // a support wider than the tile, or too few records to pay for it: tap by tap
       for (; seg; seg &= seg - 1) {
         const int src = __ffs(seg) - 1;
         const float2 *const taps = cfd + __shfl_sync(0xffffffffu, rec.g.cfoff, src);
         const float2 s = make_float2(__shfl_sync(0xffffffffu, rec.stokes[0].x, src),
                                      __shfl_sync(0xffffffffu, rec.stokes[0].y, src));
-        const size_t at = ((size_t)(band * f.npol) * f.ny + __shfl_sync(0xffffffffu, by, src)) * f.nx +
+        const int b = BLOCKS || !BANDS ? band : __shfl_sync(0xffffffffu, rec.gridchan, src);
+        const size_t at = ((size_t)(b * f.npol) * f.ny + __shfl_sync(0xffffffffu, by, src)) * f.nx +
                           __shfl_sync(0xffffffffu, bx, src);
         for (int t = lane; t < ((S * S + 31) & ~31); t += 32) {
           const bool on = t < S * S;
@@ -586,10 +605,11 @@ struct ScatterSmem<1, SLOTS> {
 
 // The warp's records onto facet f.  sm: the warp's own, cleared once (clear) before the first call.  ACC:
 // facets may have FP64 accumulators (several planes only, where that code costs the other path registers).
-template <int NPOL, int SLOTS, bool CONJ = false, bool BLOCKS = false, bool ACC = !CONJ>
+// BANDS: facets may have several bands (one plane only).
+template <int NPOL, int SLOTS, bool CONJ = false, bool BLOCKS = false, bool ACC = !CONJ, bool BANDS = true>
 __device__ __forceinline__ void scatter(const GridRecord<NPOL> &rec, const ddfg_facet &f, int npol_used,
                                         ScatterSmem<NPOL, SLOTS> &sm, int lane) {
-  if constexpr (NPOL == 1) scatter_tile<SLOTS, CONJ, BLOCKS>(rec, f, sm.tile, lane);
+  if constexpr (NPOL == 1) scatter_tile<SLOTS, CONJ, BLOCKS, BANDS>(rec, f, sm.tile, lane);
   else scatter_torus<NPOL, SLOTS, CONJ, BLOCKS, ACC>(rec, f, npol_used, sm.torus, lane);
 }
 

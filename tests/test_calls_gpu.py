@@ -235,3 +235,26 @@ def test_runs_reach_the_accumulator_in_fp64(kw):
     on = want != 0
     got = g.grid.cpu().numpy().astype(np.complex128)[on]
     assert np.sqrt(np.mean(np.abs(got / want[on] - 1) ** 2)) < 4e-8
+
+
+@pytest.mark.parametrize("stokes", [(1,), (1, 2)], ids=["i", "iq"])
+@pytest.mark.parametrize("kw", [dict(nchan=600, nband=600), dict(nchan=1600, nband=1500),
+                                dict(nchan=5000, bda_mode=1, dphi=0.5), dict(nchan=7000, bda_mode=1, dphi=0.5)],
+                         ids=["600bands", "1500bands", "5000ch", "7000ch"])
+def test_sums_of_many_bands_and_channels(kw, stokes):
+    """Weight sums in one copy that the warps of a CTA share, and per-channel Jones sums beside the tiles of
+    twelve warps.  FP64 sums of FP32 weights: 1e-12, times FP32 Jones weights: 1e-6."""
+    c = cases.make_case(seed=67, nant=4, ntimes=3, ncorr=4, npix=63, cell_arcsec=8.0, nw=2, flag_frac=0.1,
+                        stokes_ids=stokes, **kw)
+    cases.add_jones(c, nt=2, nd=2, mode=1)
+    want = cases.run_fp64_grid(c)
+    vs, fg, jd = cases._gpu_objs(c)
+    pol = D.make_pol(c.corr_ids, c.stokes_ids)
+    fs = [dataclasses.replace(fg, **{k: torch.zeros_like(getattr(fg, k)) for k in
+                                     ("grid", "sumwt", "sumjones", "sumjones_chan")}) for _ in range(3)]
+    D.grid(vs, fs, pol, jd, batch=D.Batch.create())
+    for f in fs:
+        assert cases.rel_rms(f.grid.cpu().numpy(), want["grid"]) < 1e-6
+        np.testing.assert_allclose(f.sumwt.cpu().numpy(), want["sumwt"], rtol=1e-12)
+        np.testing.assert_allclose(f.sumjones.cpu().numpy(), want["sumjones"], rtol=1e-6)
+        np.testing.assert_allclose(f.sumjones_chan.cpu().numpy(), want["sumjones_chan"], rtol=1e-6)
