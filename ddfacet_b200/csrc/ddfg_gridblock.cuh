@@ -402,8 +402,10 @@ __device__ __forceinline__ void warp_add_single_sums(const ddfg_vis &vs, const d
 // Channels up to which the single-visibility gridder keeps the per-channel Jones sums in shared
 // memory.  Straight to global memory, 32 neighbouring channels are 16 sectors a stripe and facet and
 // a shared copy (4 KB a facet at 256 channels) would cost the tile its room; with few channels every
-// warp of the GPU adds to the same few sectors (16 channels, one facet, 340,000 visibilities: 230 us
-// a call without shared copies, most of it waiting there).
+// warp of the GPU adds to the same few sectors.  Shared and global, us a call on 1, 4 and 25 facets
+// (4.8, 4.8 and 1.2-4.8 M visibilities): 64 channels 744, 2402, 3919 and 1502, 2418, 3919; 128 channels
+// 634, 1930, 3220 and 703, 1905, 3159; 200 channels 605, 1856, 3348 and 601, 1824, 3240; 256 channels 591,
+// 1755, 3845 and 620, 1736, 3642; 1024 channels 734, 2370, 14837 and 718, 2045, 11840.
 constexpr int kSharedChannels = 128;
 
 // Visibilities of block b (rows x channels, flagged ones included).
