@@ -100,12 +100,15 @@ __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ long long lrint_d(double x) { return __double2ll_rn(x); }
 
-// exp(i * 2*pi * turns): FP64 range reduction, FP32 sincospi of the fraction.
+// exp(i * 2*pi * turns): FP64 range reduction, FP32 sincospi of the fraction, and what the fraction's
+// rounding to FP32 turns away (4e-8 RMS, as much as all other roundings of a gridded visibility) put back
+// to first order.
 __device__ __forceinline__ float2 phasor_turns(double turns) {
-  double frac = turns - rint(turns);
+  const double frac = turns - rint(turns);
+  const float f = (float)frac, rest = (float)(frac - (double)f) * (float)(2. * kPi);
   float s, c;
-  sincospif(2.0f * (float)frac, &s, &c);
-  return make_float2(c, s);
+  sincospif(2.0f * f, &s, &c);
+  return make_float2(fmaf(-rest, s, c), fmaf(rest, c, s));
 }
 
 // ----------------------------------------------------------------------------------------
