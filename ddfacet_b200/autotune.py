@@ -23,6 +23,14 @@ from . import device as D
 
 GRID_CANDIDATES: List[dict] = [dict(facets_per_pack=p, stripes_per_item=s) for p in (8, 16, 32) for s in (0, 16)]
 DEGRID_CANDIDATES: List[dict] = [dict(facets_per_pack=p, stripes_per_item=s) for p in (16, 32, 0) for s in (0, 16)]
+SCHEDULE = 2  # part of the cache key: what the fields of a candidate mean to the library's scheduler
+
+
+def candidates(single: bool, grid: bool) -> List[dict]:
+    """The schedules to time for a map: chunks of 64 (the library's own for single visibilities) and of
+    16 stripes (its own for averaged blocks)."""
+    out = GRID_CANDIDATES if grid else DEGRID_CANDIDATES
+    return out if single else [dict(c, stripes_per_item=64 if c["stripes_per_item"] else 0) for c in out]
 
 
 def _cache_path() -> str:
@@ -32,13 +40,18 @@ def _cache_path() -> str:
 
 def workload_key(vs: D.VisData, facets: Sequence[D.FacetGrid], pol, jones: Optional[D.JonesData]) -> str:
     """Hash of what the best schedule depends on: grid sizes, facet count, block count (rounded to a
-    power of two), channels, correlations, Stokes planes, single-visibility map, supports, Jones mode,
-    FP64 accumulation, large-block list and the GPU."""
+    power of two), channels, correlations, Stokes planes, single-visibility map, supports, FP64
+    accumulation, large-block list, what the choice of kernel reads (smearing, Jones terms and how they
+    are used), the scheduler and the GPU."""
     sizes = sorted({tuple(f.grid.shape) for f in facets})
     nb = max(1, int(vs.nblocks))
-    desc = dict(sizes=sizes, nfacets=len(facets), nblocks_log2=nb.bit_length(), nchan=int(vs.vis.shape[1]),
-                ncorr=int(vs.vis.shape[2]), npol=int(pol.npol), single=int(vs.single_vis_blocks),
-                sup=max(int(f.cf.max_support) for f in facets), jones=0 if jones is None else int(jones.mode),
+    terms = None if jones is None else (int(jones.mode), jones.kms is not None, jones.beam is not None,
+                                        int(jones.interp_mode), int(jones.apply_amp), int(jones.apply_phase),
+                                        int(jones.scale_jones))
+    desc = dict(schedule=SCHEDULE, sizes=sizes, nfacets=len(facets), nblocks_log2=nb.bit_length(),
+                nchan=int(vs.vis.shape[1]), corr=list(pol.corr_ids)[:int(pol.ncorr)],
+                stokes=list(pol.stokes_ids)[:int(pol.npol)], single=int(vs.single_vis_blocks),
+                sup=max(int(f.cf.max_support) for f in facets), jones=terms, smear=vs.uvw_dt is not None,
                 acc64=any(f.grid_acc is not None for f in facets), large=vs.large_blocks is not None,
                 gpu=torch.cuda.get_device_name(vs.vis.device))
     return hashlib.sha1(json.dumps(desc, sort_keys=True, default=str).encode()).hexdigest()[:16]
@@ -140,7 +153,8 @@ def tune(vs: D.VisData, facets_grid: Sequence[D.FacetGrid], facets_model: Sequen
                for f in facets_grid]
     table: Dict[str, list] = {"grid": [], "degrid": []}
     best_g, best_gms = None, float("inf")
-    for cand in (grid_candidates or GRID_CANDIDATES):
+    single = bool(vs.single_vis_blocks)
+    for cand in (grid_candidates or candidates(single, True)):
         b = D.Batch.create(dev, **cand)
         ms = _time(lambda: D.grid(sv, scratch, pol, jones, batch=b))
         table["grid"].append((cand, round(ms, 3)))
@@ -152,7 +166,7 @@ def tune(vs: D.VisData, facets_grid: Sequence[D.FacetGrid], facets_model: Sequen
     del scratch
     sd = dataclasses.replace(sv, vis=vs.vis.clone())
     best_d, best_dms = None, float("inf")
-    for cand in (degrid_candidates or DEGRID_CANDIDATES):
+    for cand in (degrid_candidates or candidates(single, False)):
         b = D.Batch.create(dev, **cand)
         ms = _time(lambda: D.degrid(sd, list(facets_model), pol, jones, batch=b))
         table["degrid"].append((cand, round(ms, 3)))
