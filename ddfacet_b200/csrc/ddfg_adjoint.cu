@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(256, 2) jones_grad_single_i(const ddfg_vis vs,
         const bool valid = in.valid && in.gridchan < f.nband &&
                            geometry_i(f, dadd(in.U, dmul(in.W, f.cu)), dadd(in.V, dmul(in.W, f.cv)), in.W, in.recip, geo);
         float2 t;
-        gather<1, SLOTS>(valid, geo, in.gridchan, sf[fi], ws, lane, &t);
+        gather<1, SLOTS, false>(valid, geo, in.gridchan, sf[fi], ws, lane, &t);
         t = cmul(t, phasor_turns(in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * f.n0m1) * kInvC));
         M2 A;
 #pragma unroll
@@ -795,7 +795,9 @@ int ddfg_launch_jones_grad(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_
     const int f0 = (int)(((long long)ip * nfacets) / npacks);
     FacetPackD pack;
     pack.n = (int)(((long long)(ip + 1) * nfacets) / npacks) - f0;
-    if (adjoint_is_i(vs, js, policy)) {
+    bool far = false;
+    for (int i = 0; i < pack.n; ++i) far = far || far_bands(facets[f0 + i]);
+    if (!far && adjoint_is_i(vs, js, policy)) {
       const int rc = slots == 2 ? launch_i<2>(vs, js, facets + f0, pack.n, g, stream)
                                 : launch_i<4>(vs, js, facets + f0, pack.n, g, stream);
       if (rc) return rc;

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256, SLOTS == 2 ? 3 : 2)
         const bool valid = in.valid && in.gridchan < f.nband &&
                            geometry_i(f, dadd(in.U, dmul(in.W, f.cu)), dadd(in.V, dmul(in.W, f.cv)), in.W, in.recip, g);
         float2 t;
-        gather<1, SLOTS>(valid, g, in.gridchan, sf[fi], ws, lane, &t);
+        gather<1, SLOTS, false>(valid, g, in.gridchan, sf[fi], ws, lane, &t);
         t = cmul(t, phasor_turns(in.nu * (in.U * f.l0 + in.V * f.m0 + in.W * f.n0m1) * kInvC));
         if (use) {
           const JonesProduct<false> jp = jones_for<false>(js, use, ju, in.valid, at, f.jones_dir, keep + fi, lane);
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(256, 2) degrid_block_i(const ddfg_vis vs, cons
           valid = geometry_i(f, m.u, m.v, m.w, m.recip, g);
         }
         float2 t;
-        gather<1, SLOTS>(valid, g, d.gridchan, sf[fi], ws, lane, &t);
+        gather<1, SLOTS, false>(valid, g, d.gridchan, sf[fi], ws, lane, &t);
         bool apply = valid;
         if (large) {
           apply = __shfl_sync(0xffffffffu, valid, 0);
@@ -333,8 +333,9 @@ template <int NP, int SL>
 int launch_degrid_table(const ddfg_vis *vs, const ddfg_jones *js, const FacetTable &tab, const DegridParams &dp,
                         Sched sc, const ddfg_batch *batch, bool &zeroed, int counters, cudaStream_t stream) {
   const bool single = vs->single_vis_blocks != 0;
-  const bool stokes_i = NP == 1 && dp.policy == D_DIAG_FROM_I && !vs->uvw_dt && jones_as_stored(js) &&
-                        (single || js->mode != 2);
+  bool stokes_i = NP == 1 && dp.policy == D_DIAG_FROM_I && !vs->uvw_dt && jones_as_stored(js) &&
+                  (single || js->mode != 2);
+  for (int i = 0; i < sc.nfacets; ++i) stokes_i = stokes_i && !far_bands(tab.f[i]);
   const size_t smem = stokes_i ? 8 * sizeof(GatherSmem<1>) + (sizeof(ddfg_facet) + sizeof(FacetI) +
                                                               (single ? 8 * sizeof(JonesProduct<false>) : 0)) *
                                                                  (size_t)sc.max_pack

@@ -16,6 +16,11 @@
 
 namespace ddfg {
 
+// Cells of a facet's bands together do not fit an int32 index: records are then taken band by band.
+__host__ __device__ __forceinline__ bool far_bands(const ddfg_facet &f) {
+  return f.nband > 1 && (int64_t)f.nband * f.npol * f.ny * f.nx > 0x7fffffff;
+}
+
 // Taps a lane and pass for the largest support of a launch: supports up to 8 fit two; wider ones take
 // four, or two where the Stokes planes multiply the registers.
 inline int tap_slots(int max_support, int npol) { return max_support <= 8 || npol > 2 ? 2 : 4; }
@@ -384,8 +389,8 @@ struct alignas(16) TorusSmem {
 // One pass of the torus over n records (n a multiple of four) of support S, into the float32 grid.
 template <int NPOL, int SLOTS, bool CONJ>
 __device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int S, int first,
-                                           const ddfg_facet &f, int npol_used, int lane) {
-  float2 *const grid = (float2 *)f.grid;
+                                           const ddfg_facet &f, size_t origin, int npol_used, int lane) {
+  float2 *const grid = (float2 *)f.grid + origin;
   const float2 *const cfd = (const float2 *)f.cf_data;
   const int nx = f.nx;
   const size_t plane = (size_t)f.nx * f.ny;
@@ -459,10 +464,10 @@ __device__ __forceinline__ void torus_pass(const TorusSmem<NPOL> &sm, int n, int
 // 15.8 ms, 5.2 ms this way; with both kinds of grid in one loop the float32 one takes 2.47 ms instead of
 // 1.25).
 template <int NPOL, bool RUN64>
-__device__ __noinline__ void torus_acc(const TorusSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, int npol_used,
-                                       int lane) {
+__device__ __noinline__ void torus_acc(const TorusSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, size_t origin,
+                                       int npol_used, int lane) {
   using Sum = typename std::conditional<RUN64, double2, float2>::type;
-  double *const acc = (double *)f.grid_acc;
+  double *const acc = (double *)f.grid_acc + 2 * origin;
   const float2 *const cfd = (const float2 *)f.cf_data;
   const int nx = f.nx;
   const size_t plane = (size_t)f.nx * f.ny;
@@ -541,9 +546,12 @@ __device__ __forceinline__ void scatter_torus(const GridRecord<NPOL> &rec, const
                                               TorusSmem<NPOL> &sm, int lane) {
   unsigned mask = __ballot_sync(0xffffffffu, rec.valid);
   bool mixed = false;  // several supports
+  const bool far = far_bands(f);
   while (mask) {
-    const int S = __shfl_sync(0xffffffffu, rec.g.S, __ffs(mask) - 1);
-    const bool mine = rec.valid && rec.g.S == S;
+    const int lead = __ffs(mask) - 1, S = __shfl_sync(0xffffffffu, rec.g.S, lead);
+    const int band = far ? __shfl_sync(0xffffffffu, rec.gridchan, lead) : 0;
+    const size_t origin = (size_t)band * f.npol * f.ny * f.nx;
+    const bool mine = rec.valid && rec.g.S == S && (!far || rec.gridchan == band);
     const unsigned sub = __ballot_sync(0xffffffffu, mine);
     mixed = mixed || sub != mask;
     mask &= ~sub;
@@ -552,7 +560,7 @@ __device__ __forceinline__ void scatter_torus(const GridRecord<NPOL> &rec, const
     if (mine) {
       const int bx = rec.g.locx - rec.g.sup, by = rec.g.locy - rec.g.sup;
       const unsigned magic = torus_magic(S);
-      base = ((rec.gridchan * f.npol) * f.ny + by) * f.nx + bx;
+      base = (((rec.gridchan - band) * f.npol) * f.ny + by) * f.nx + bx;
       mod = torus_mod(bx, S, magic) | torus_mod(by, S, magic) << 8;
       cfo = rec.g.cfoff;
       const int at = __popc(sub & ((1u << lane) - 1u));
@@ -574,13 +582,13 @@ __device__ __forceinline__ void scatter_torus(const GridRecord<NPOL> &rec, const
     }
     __syncwarp();
     if (ACC && f.grid_acc) {
-      if (BLOCKS || S > 16 || mixed) torus_acc<NPOL, true>(sm, n, S, f, npol_used, lane);
-      else torus_acc<NPOL, false>(sm, n, S, f, npol_used, lane);
+      if (BLOCKS || S > 16 || mixed) torus_acc<NPOL, true>(sm, n, S, f, origin, npol_used, lane);
+      else torus_acc<NPOL, false>(sm, n, S, f, origin, npol_used, lane);
     } else if (SLOTS > 2 && S <= 8) {
-      torus_pass<NPOL, 2, CONJ>(sm, n4, S, 0, f, npol_used, lane);
+      torus_pass<NPOL, 2, CONJ>(sm, n4, S, 0, f, origin, npol_used, lane);
     } else {
       for (int first = 0; first < S * S; first += 32 * SLOTS)
-        torus_pass<NPOL, SLOTS, CONJ>(sm, n4, S, first, f, npol_used, lane);
+        torus_pass<NPOL, SLOTS, CONJ>(sm, n4, S, first, f, origin, npol_used, lane);
     }
     __syncwarp();
   }
@@ -665,7 +673,8 @@ __device__ __forceinline__ void gather_store(GatherSmem<NPOL> &sm, const float2 
 
 // Sums n records (a multiple of four) of support S <= 8: a run's model cells stay in registers.
 template <int NPOL>
-__device__ __forceinline__ void gather_narrow(GatherSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, int lane) {
+__device__ __forceinline__ void gather_narrow(GatherSmem<NPOL> &sm, int n, int S, const ddfg_facet &f,
+                                              const float2 *grid, int lane) {
   constexpr int GROUP = NPOL == 1 ? 4 : NPOL == 2 ? 4 : 2;  // records in flight
   const size_t plane = (size_t)f.nx * f.ny;
   bool on[2];
@@ -675,7 +684,7 @@ __device__ __forceinline__ void gather_narrow(GatherSmem<NPOL> &sm, int n, int S
   for (int k = 0; k < 2; ++k) {
     const int t = lane + 32 * k, sy = tap_row(t, S);
     on[k] = t < S * S;
-    cell[k] = (const float2 *)f.grid + (sy * f.nx + t - sy * S);
+    cell[k] = grid + (sy * f.nx + t - sy * S);
 #pragma unroll
     for (int p = 0; p < NPOL; ++p) held[p][k] = czero();
 #pragma unroll
@@ -720,11 +729,11 @@ __device__ __forceinline__ void gather_narrow(GatherSmem<NPOL> &sm, int n, int S
 // The same for any support: four records at a time over all their taps, 32 SLOTS a round, so that a
 // record still costs one partial sum a lane.  Records of a round on one origin share its cells.
 template <int NPOL, int SLOTS>
-__device__ __forceinline__ void gather_wide(GatherSmem<NPOL> &sm, int n, int S, const ddfg_facet &f, int lane) {
+__device__ __forceinline__ void gather_wide(GatherSmem<NPOL> &sm, int n, int S, const ddfg_facet &f,
+                                            const float2 *grid, int lane) {
   constexpr int GROUP = NPOL <= 2 ? 4 : 2;
   const size_t plane = (size_t)f.nx * f.ny;
   const float2 *const cfd = (const float2 *)f.cf_data + lane;
-  const float2 *const grid = (const float2 *)f.grid;
   const int row0 = tap_row(lane, S), col0 = lane - row0 * S, drow = tap_row(32, S), dcol = 32 - drow * S;
   for (int i = 0; i < n; i += GROUP) {
     int2 q[GROUP];
@@ -771,29 +780,34 @@ __device__ __forceinline__ void gather_wide(GatherSmem<NPOL> &sm, int n, int S, 
 }
 
 // The sums over every valid record's taps on facet f (degridder.h:202-212); the sum of lane r's
-// record ends in its mine[].  sm: the warp's own.  Must be called by all 32 lanes.
-template <int NPOL, int SLOTS>
+// record ends in its mine[].  sm: the warp's own.  Must be called by all 32 lanes.  FAR: the facet may have
+// far_bands (the Stokes I kernels do without: 2 to 3 % of degrid_single_i).
+template <int NPOL, int SLOTS, bool FAR = true>
 __device__ __forceinline__ void gather(bool valid, const BlockGeom &g, int gridchan, const ddfg_facet &f,
                                        GatherSmem<NPOL> &sm, int lane, float2 *mine) {
 #pragma unroll
   for (int p = 0; p < NPOL; ++p) mine[p] = czero();
   unsigned mask = __ballot_sync(0xffffffffu, valid);
+  const bool far = FAR && far_bands(f);
   while (mask) {
-    const int S = __shfl_sync(0xffffffffu, g.S, __ffs(mask) - 1);
-    const bool own = valid && g.S == S;
+    const int lead = __ffs(mask) - 1, S = __shfl_sync(0xffffffffu, g.S, lead);
+    const int band = far ? __shfl_sync(0xffffffffu, gridchan, lead) : 0;
+    const float2 *const grid = (const float2 *)f.grid + (size_t)band * f.npol * f.ny * f.nx;
+    const bool own = valid && g.S == S && (!far || gridchan == band);
     const unsigned sub = __ballot_sync(0xffffffffu, own);
     mask &= ~sub;
     const int n = __popc(sub), n4 = (n + 3) & ~3;
     const int at = __popc(sub & ((1u << lane) - 1u));
     if (own) {
-      const int2 q = make_int2(((gridchan * f.npol) * f.ny + g.locy - g.sup) * f.nx + g.locx - g.sup, g.cfoff);
+      const int2 q = make_int2((((gridchan - band) * f.npol) * f.ny + g.locy - g.sup) * f.nx + g.locx - g.sup,
+                               g.cfoff);
       sm.rec[at] = q;
       if (at == n - 1)  // copies of the last record fill the last group of four
         for (int j = n; j < n4; ++j) sm.rec[j] = q;
     }
     __syncwarp();
-    if (S <= 8) gather_narrow<NPOL>(sm, n4, S, f, lane);
-    else gather_wide<NPOL, SLOTS>(sm, n4, S, f, lane);
+    if (S <= 8) gather_narrow<NPOL>(sm, n4, S, f, grid, lane);
+    else gather_wide<NPOL, SLOTS>(sm, n4, S, f, grid, lane);
     if (own) {
 #pragma unroll
       for (int p = 0; p < NPOL; ++p) mine[p] = sm.out[at][p];

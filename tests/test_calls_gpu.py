@@ -275,3 +275,36 @@ def test_phasor_rounding():
     on = want != 0
     assert on.mean() > 0.9
     assert np.sqrt(np.mean(np.abs(got[on] / want[on] - 1) ** 2)) < 5e-8
+
+
+@pytest.mark.parametrize("stokes,n", [((1,), 33000), ((1, 2), 23200)], ids=["i", "iq"])
+def test_bands_beyond_two_billion_cells(stokes, n):
+    """Two bands of a grid of more than 2^31 cells: the second is gridded and degridded as the only band of
+    a grid of half the size is (float32 grids: another order of the additions, 1e-6)."""
+    c = cases.make_case(seed=69, nant=7, ntimes=6, nchan=8, ncorr=4, npix=127, cell_arcsec=5.0, nw=2, stokes_ids=stokes)
+    vs, fg, _ = cases._gpu_objs(c)
+    incr = tuple(x * c.npix / n for x in c.incr)  # the same footprints about the middle of the grid
+    pol = D.make_pol(c.corr_ids, c.stokes_ids)
+    npol, lo, hi = len(stokes), n // 2 - 100, n // 2 + 100
+    model = _randn((npol, hi - lo, hi - lo), 5)
+    got = {}
+    for nband in (1, 2):
+        v = dataclasses.replace(vs, chan_map=torch.full_like(vs.chan_map, nband - 1))
+        grid = torch.zeros((nband, npol, n, n), dtype=torch.complex64, device="cuda")
+        f = dataclasses.replace(fg, grid=grid, incr=incr, sumwt=None, sumjones=None, sumjones_chan=None, grid_acc=None)
+        out = []
+        for acc in (None, torch.zeros(grid.shape, dtype=torch.complex128, device="cuda")):
+            D.grid(v, [dataclasses.replace(f, grid_acc=acc)], pol)
+            out.append(grid[-1, :, lo:hi, lo:hi].clone())
+            grid[-1, :, lo:hi, lo:hi] = 0
+            assert not torch.view_as_real(grid).any()  # nothing elsewhere
+            del acc
+        grid[-1, :, lo:hi, lo:hi] = model
+        d = dataclasses.replace(v, vis=torch.zeros_like(v.vis))
+        D.degrid(d, [f], pol)
+        got[nband] = [*out, d.vis]
+        del f, grid
+        torch.cuda.empty_cache()
+    for a, b in zip(got[2], got[1]):
+        assert torch.count_nonzero(torch.view_as_real(b)) > 0
+        assert _rms(a, b) < 1e-6
