@@ -681,9 +681,14 @@ def run_gpu(args):
         except Exception as e:  # reported, not allowed to drop the measurement
             out["dropin"] = {"error": repr(e)[:300]}
         if args.workload in WORKLOADS:
-            mv, cores, sample = cpu_reference(args.workload)
-            out["cpu_baseline"] = {"value": round(mv, 4), "unit": UNIT, "cores": cores, "kind": "reference",
-                                   "sample": sample}
+            from oracle import ref
+
+            if ref.available():
+                mv, cores, sample = cpu_reference(args.workload)
+                out["cpu_baseline"] = {"value": round(mv, 4), "unit": UNIT, "cores": cores, "kind": "reference",
+                                       "sample": sample}
+            else:
+                out["cpu_baseline"] = {"unavailable": "oracle/_ref not built (oracle/build_ref.sh)"}
     if rank == 0:
         print(json.dumps(out), flush=True)
 
