@@ -13,7 +13,7 @@
 // Warps meet at a barrier only between packs: with a barrier per item of a CTA a tenth of the
 // warps' time (a sixth on averaged blocks) went into waiting for its slowest warp; with small
 // items handed to single warps instead, neighbouring stripes fell on different SMs and half of the
-// L1 hits were lost (averaged degridding 28 ms against 24 ms).  The pack-major order keeps the grids of
+// L1 hits were lost (averaged degridding a sixth slower).  The pack-major order keeps the grids of
 // one pack at a time live in L2.
 #pragma once
 #include "ddfg_common.cuh"

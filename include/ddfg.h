@@ -70,12 +70,13 @@ typedef struct ddfg_facet {
   double *sumjones;            /* [2][nband]      (LJones[17])                            */
   double *sumjones_chan;       /* [2][nchan]      (LJones[18])                            */
   /* FP64 accumulation (optional; NULL = float32 atomic additions into grid).  A complex128 buffer
-   * [nband][npol][ny][nx], all zero on entry: ddfg_grid / ddfg_grid_batched add every tap product
-   * into it with FP64 atomics instead of into grid, and at the end of the call add it into grid
-   * (one float32 rounding per cell: grid = fl(grid + acc)) and zero it again.  The grid then holds
-   * the float32 rounding of the call's sum instead of the sum of ~10^4-10^6 successively rounded
-   * float32 additions per cell, as the reference's FP64 products would give if its grid were
-   * wider (gridder.h:360-362 adds them into the float grid one by one). */
+   * [nband][npol][ny][nx], all zero on entry: ddfg_grid / ddfg_grid_batched add the tap products into
+   * it in FP64 instead of into grid (runs of neighbouring visibilities of one support up to 16 are
+   * summed in FP32 first), and at the end of the call add it into grid (one float32 rounding per
+   * cell: grid = fl(grid + acc)) and zero it again.  The grid then holds the float32 rounding of the
+   * call's sum instead of the sum of ~10^4-10^6 successively rounded float32 additions per cell, as
+   * the reference's FP64 products would give if its grid were wider (gridder.h:360-362 adds them into
+   * the float grid one by one).  The other calls do not read or write it. */
   void *grid_acc;
 } ddfg_facet;
 
@@ -305,8 +306,9 @@ size_t ddfg_batch_workspace_size(void);
 
 /* ddfg_grid as one persistent, scheduled launch per DDFG_TABLE_FACETS facets (see
  * ddfg_batch): same inputs, outputs and checks.  The work queue balances uneven facets and
- * blocks (averaged BDA blocks of very different sizes) across the GPU; every call first resets
- * its counters (one cudaMemsetAsync), so the call can be captured in a CUDA graph.  Replaces the
+ * blocks (averaged BDA blocks of very different sizes) across the GPU; a call that uses it first
+ * resets its counters (one cudaMemsetAsync; calls of less than two stripes a warp go without), so
+ * the call can be captured in a CUDA graph.  Replaces the
  * per-facet gridding jobs of ClassFacetMachine (ClassFacetMachine.py:1574-1592). */
 int ddfg_grid_batched(const ddfg_vis *vs, const ddfg_jones *js, const ddfg_pol *pol, const ddfg_facet *facets,
                       int nfacets, int dopsf, const ddfg_batch *batch, void *stream);
