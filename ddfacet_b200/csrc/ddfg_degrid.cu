@@ -18,11 +18,12 @@
 // serialises the same update across facet processes with named semaphores (degridder.h:236-263).
 // Single-visibility maps sum the pack's predictions in registers and subtract once per pack.
 //
-// What bounds them (256 channels, 16 facets a pack, 310 M facet-visibilities): the L1 data path (73 %
-// of its wavefronts: four for a record's taps, five when its model cells change, four for its lane
-// partials) and issue (63 %, 30 instructions a record); 28.3 ms before records went through shared
-// memory, runs kept their model cells and Stokes I had kernels of its own (ddfg_single.cuh), 23.9 ms
-// now.  Averaged blocks (9 uneven facets): 24.3 ms to 15.2 ms, on the latency of the block walks.
+// What bounds them (256 channels, 16 facets a pack): the latency of taps and model cells from L2 (half of
+// the cycles between issues), the L1 data path (67 %: four wavefronts for a record's taps, five when its
+// model cells change, four for its lane partials) and issue (57 %, 53 instructions a record) together;
+// 310 M facet-visibilities took 28.3 ms before records went through shared memory, runs kept their model
+// cells and Stokes I had kernels of its own (ddfg_single.cuh), 24.4 ms since.  Averaged blocks (9 uneven
+// facets): 24.3 ms to 15.2 ms, on the latency of the block walks.
 #include <cuda_runtime.h>
 
 #include "ddfg_common.cuh"

@@ -26,8 +26,8 @@
 //
 // What bounds them (256 channels, 25 facets of 1485^2, 310 M facet-visibilities, FP64 sums): 38.5 ms
 // with a reduction per tap and run, on the FP64 reduction rate of L2 (16 sectors a record, 125 G
-// sectors/s); now 26.4 ms at 48 instructions and 3.8 sectors a record, on instruction issue (51 %)
-// and the shared-memory / L1 data path (57 %) together -- 24 warps an SM instead of 16 change
+// sectors/s); with tiles 26.3 ms at 52 instructions and 2.4 sectors a record, on instruction issue (50 %)
+// and the shared-memory / L1 data path (61 %) together -- 24 warps an SM instead of 16 change
 // nothing.  64 channels, 735^2: 16.7 ms to 8.1 ms.
 #include <cuda_runtime.h>
 

@@ -263,12 +263,11 @@ class FacetGrid:
     grid_acc: Optional[torch.Tensor] = None     # complex128 like grid: FP64 accumulation (all zero)
 
     def with_fp64_accumulation(self) -> "FacetGrid":
-        """This facet with an FP64 accumulator (ddfg_facet.grid_acc): gridding adds every tap
-        product into it with FP64 atomics and, at the end of each call, adds it into the float32
-        grid (one rounding per cell) and zeroes it, so each call adds the correctly rounded sum of
-        its contributions.  The atomics do not return a value, so the call costs little more than
-        with float32 sums (10-16 % on the combined at-scale chunk, more when the accumulators of a
-        pack overflow L2 badly), and the accumulator takes twice the grid's memory."""
+        """This facet with an FP64 accumulator (ddfg_facet.grid_acc): gridding sums its tap products in
+        FP64 and, at the end of each call, adds them into the float32 grid (one rounding per cell), so
+        each call adds the rounded sum of its contributions.  The call costs little more than with
+        float32 sums (5 % on the combined at-scale chunk, more when the accumulators of a pack overflow
+        L2 badly), and the accumulator takes twice the grid's memory."""
         if self.grid_acc is None:
             self.grid_acc = torch.zeros(self.grid.shape, dtype=torch.complex128, device=self.grid.device)
         return self
