@@ -308,3 +308,21 @@ def test_bands_beyond_two_billion_cells(stokes, n):
     for a, b in zip(got[2], got[1]):
         assert torch.count_nonzero(torch.view_as_real(b)) > 0
         assert _rms(a, b) < 1e-6
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(bda_mode=1, dphi=0.6), dict(nchan=130)], ids=["single", "bda", "130ch"])
+def test_one_correlation_against_fp64(kw):
+    """One correlation goes to the general gridding kernels and to the Stokes I degridder.  Grids and
+    predictions carry some ten FP32 roundings, 3e-7 at most together: 1e-6; weight sums 1e-12, sums with
+    FP32 Jones weights 1e-6."""
+    c = cases.make_case(**{**dict(seed=70, nant=7, ntimes=10, nchan=9, ncorr=1, npix=127, cell_arcsec=5.0, nw=3, nband=2,
+                                  flag_frac=0.1), **kw})
+    cases.add_jones(c, nt=2, nd=2, mode=1, nch=2)
+    want = cases.run_fp64_grid(c)
+    got = cases.run_gpu_grid(c, batched=True, fp64_acc=True)
+    assert cases.rel_rms(got["grid"], want["grid"]) < 1e-6
+    np.testing.assert_allclose(got["sumwt"], want["sumwt"], rtol=1e-12)
+    np.testing.assert_allclose(got["sumjones"], want["sumjones"], rtol=1e-6)
+    np.testing.assert_allclose(got["sumjones_chan"], want["sumjones_chan"], rtol=1e-6)
+    model = want["grid"].astype(np.complex64)
+    assert cases.rel_rms(cases.run_gpu_degrid(c, model, batched=True), cases.run_fp64_degrid(c, model)) < 1e-6
